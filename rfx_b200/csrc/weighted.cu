@@ -35,17 +35,11 @@
 namespace rfx {
 namespace {
 
-constexpr int WR_THREADS = 128;
-constexpr int WR_WINDOW = 4096;  // columns per CTA: two FP64 accumulators each (64 KB)
-
-__device__ __forceinline__ int lower_bound_memb(const int32_t* __restrict__ a, int lo, int hi, int v) {
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(a + mid) < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
+// Weighted pair-sum rows: columns of a window (two FP64 sums each; 1,024 = 16
+// KB, 13 warps an SM: 1.32 ms at n = 5,000 / 500 trees, 512 took 1.66 and
+// 2,048 1.59) and ranges whose loads are in flight together.
+constexpr int WR_WINDOW = 1024;
+constexpr int WR_BATCH = 4;
 
 // tnodewt: one thread per (sample, tree) of the in-bag samples; integer sums
 // (exact, so the order of the float sums of the reference does not matter).
@@ -142,95 +136,235 @@ __global__ void key_mass_kernel(const int64_t* __restrict__ segbase, const int32
 
 enum { WR_CASEWISE = 0, WR_RFGAP = 1, WR_PLAIN = 2 };
 
-// One CTA per (row i, window of WR_WINDOW columns); trees in order.  For every
-// tree, the row's key k (2 * node + in-bag) gives the opposite key's members,
-// cut to the window's columns > i.
-//   i OOB (k even):   accA[j] += w(j) for the in-bag members j
-//   i in-bag (k odd): accB[j] += w(i) for the OOB members j
+// One row's part of one tree: the members of the opposite bag status in the
+// row's leaf with ids above the row's (start within the tree's member list,
+// count; the top bit of `len` marks an in-bag row), and the row's factor:
+//   out-of-bag row: the in-bag key's mass m (case-wise) or 1 / m (RF-GAP);
+//   in-bag row: the finished weight of the row in its leaf.
+struct __align__(16) WRange {
+    int lo;
+    unsigned len;
+    double w;
+};
+constexpr unsigned WR_INBAG = 0x80000000u;
+
+// Range table of the rows [i0, i1), row-major (T entries a row), so that the
+// row kernel reads its trees' entries coalesced and does no search, mass
+// lookup or division per tree.  32 rows x 32 trees per CTA, transposed
+// through shared memory.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+weighted_ranges_kernel(const int32_t* __restrict__ key, const int64_t* __restrict__ segbase,
+                       const int32_t* __restrict__ segoff, const int32_t* __restrict__ memb,
+                       const long long* __restrict__ mass, const int32_t* __restrict__ nin, int n, int T, int i0,
+                       int i1, WRange* __restrict__ tab) {
+    __shared__ WRange tile[32][33];
+    const int ib = i0 + blockIdx.x * 32, tb = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8) {
+        const int t = tb + r, i = ib + tx;
+        WRange v{0, 0u, 0.0};
+        const int k = t < T && i < i1 ? __ldg(key + (size_t)t * n + i) : -1;
+        if (k >= 0) {
+            const int64_t sb = segbase[t];
+            const int32_t* so = segoff + sb;
+            const int32_t* mt = memb + (size_t)t * n;
+            int lo = __ldg(so + (k ^ 1)), hi = __ldg(so + (k ^ 1) + 1);
+            const int end = hi;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (__ldg(mt + mid) <= i) lo = mid + 1;
+                else hi = mid;
+            }
+            const long long m = end > lo ? mass[sb + (k | 1)] : 0;  // the in-bag key of the leaf
+            if (end > lo && (m > 0 || MODE == WR_PLAIN)) {
+                v.lo = lo;
+                v.len = (unsigned)(end - lo);
+                if ((k & 1) == 0) {
+                    v.w = MODE == WR_PLAIN ? 1.0 : MODE == WR_RFGAP ? __ddiv_rn(1.0, (double)m) : (double)m;
+                } else {
+                    const double c = (double)__ldg(nin + (size_t)t * n + i);
+                    v.len |= WR_INBAG;
+                    v.w = MODE == WR_PLAIN   ? 1.0
+                          : MODE == WR_RFGAP ? __dmul_rn(c, __ddiv_rn(1.0, (double)m))
+                                             : __ddiv_rn(c, (double)m);
+                }
+            }
+        }
+        tile[r][tx] = v;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int i = ib + r, t = tb + tx;
+        if (i < i1 && t < T) tab[(size_t)(i - i0) * T + t] = tile[tx][r];
+    }
+}
+
+// Weight of every in-bag member in member-list order (case-wise nin / mass,
+// RF-GAP nin x (1 / mass)), so that the row kernel reads it beside the member
+// instead of dividing per pair.
+template <int MODE>
+__global__ void member_weight_kernel(const int32_t* __restrict__ key, const int64_t* __restrict__ segbase,
+                                     const int32_t* __restrict__ segoff, const int32_t* __restrict__ memb,
+                                     const long long* __restrict__ mass, const int32_t* __restrict__ nin, int n,
+                                     double* __restrict__ wm) {
+    const int t = blockIdx.y;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t sb = segbase[t];
+    if (q >= __ldg(segoff + segbase[t + 1] - 1)) return;  // members without a key follow the keyed ones
+    const size_t tn = (size_t)t * n;
+    const int j = __ldg(memb + tn + q);
+    const int k = __ldg(key + tn + j);
+    if (!(k & 1)) return;
+    const double c = (double)__ldg(nin + tn + j), m = (double)mass[sb + k];
+    wm[tn + q] = MODE == WR_RFGAP ? __dmul_rn(c, __ddiv_rn(1.0, m)) : __ddiv_rn(c, m);
+}
+
+// One warp per row i.
+//   i out of bag: accA[j] += w(j) for the in-bag members j
+//   i in-bag:     accB[j] += w(i) for the out-of-bag members j
 // casewise: w(s) = nin[s] / nodesize (nodesize = mass of the in-bag key);
 //           S[i][j] = accA[j] + accB[j].
 // plain:    w = 1 (the reference's weights without use_casewise), as FP64.
 // rfgap:    w(s) = nin[s] * (1 / M), M = mass of the in-bag key;
 //           P[i][j] = (accA[j] / |S_i| + accB[j] / |S_j|) / 2, with the
 //           reference's multiplication by 1 / |S|.
-template <int MODE>
-__global__ void __launch_bounds__(WR_THREADS)
-weighted_row_kernel(const int32_t* __restrict__ key, const int64_t* __restrict__ segbase,
-                    const int32_t* __restrict__ segoff, const int32_t* __restrict__ memb,
-                    const long long* __restrict__ mass, const int32_t* __restrict__ nin,
-                    const int32_t* __restrict__ nout, int n, int T, double* __restrict__ out) {
-    extern __shared__ double wr_acc[];  // accA | accB, WR_WINDOW each
-    double* accA = wr_acc;
-    double* accB = wr_acc + WR_WINDOW;
-    const int i = blockIdx.x;
-    const int c0 = blockIdx.y * WR_WINDOW;
-    const int c1 = min(n, c0 + WR_WINDOW);
-    if (c1 <= i) return;  // every column of the window lies left of the diagonal
-    const int lo = max(c0, i + 1);
-    const int tid = threadIdx.x;
-    for (int k = tid; k < WR_WINDOW; k += WR_THREADS) {
-        accA[k] = 0.0;
-        accB[k] = 0.0;
-    }
-    __syncthreads();
-    for (int t = 0; t < T; ++t) {
-        const int k = __ldg(key + (size_t)t * n + i);
-        if (k >= 0 && lo < c1) {
-            const int64_t sb = segbase[t];
-            const int32_t* so = segoff + sb;
-            const int32_t* mt = memb + (size_t)t * n;
-            const int ok = k ^ 1;
-            int b = __ldg(so + ok), e = __ldg(so + ok + 1);
-            if (b < e) {
-                b = lower_bound_memb(mt, b, e, lo);
-                e = lower_bound_memb(mt, b, e, c1);
-            }
-            const int32_t* nt = nin + (size_t)t * n;
-            if ((k & 1) == 0) {
-                const long long m = mass[sb + ok];
-                if (m > 0 || MODE == WR_PLAIN) {
-                    const double inv = MODE == WR_RFGAP ? __ddiv_rn(1.0, (double)m) : 0.0;
-                    for (int q = b + tid; q < e; q += WR_THREADS) {
-                        const int j = __ldg(mt + q);
-                        const double c = (double)__ldg(nt + j);
-                        const double w = MODE == WR_PLAIN   ? 1.0
-                                         : MODE == WR_RFGAP ? __dmul_rn(c, inv)
-                                                            : __ddiv_rn(c, (double)m);
-                        accA[j - c0] = __dadd_rn(accA[j - c0], w);
-                    }
-                }
-            } else {
-                const long long m = mass[sb + k];
-                if (m > 0 || MODE == WR_PLAIN) {
-                    const double c = (double)__ldg(nt + i);
-                    const double w = MODE == WR_PLAIN   ? 1.0
-                                     : MODE == WR_RFGAP ? __dmul_rn(c, __ddiv_rn(1.0, (double)m))
-                                                        : __ddiv_rn(c, (double)m);
-                    for (int q = b + tid; q < e; q += WR_THREADS) {
-                        const int j = __ldg(mt + q);
-                        accB[j - c0] = __dadd_rn(accB[j - c0], w);
-                    }
-                }
-            }
-        }
-        __syncthreads();  // this tree's adds land before the next tree's
-    }
+// Every sum runs in the warp's program order, tree after tree, with no barrier.
+// The row is taken in windows of `win` columns whose sums sit in shared
+// memory; the row's ranges keep their position in the table between windows
+// (members ascend), so nothing is searched.  The warp takes 32 trees at a time
+// (lane = tree) and adds the ranges that reach into the window one after the
+// other, lanes on consecutive members: the columns of one range are distinct,
+// so no lane meets another.  The loads of the next WR_BATCH ranges are in
+// flight with the adds of the current ones.
+// PRE: the in-bag members' weights come from member_weight_kernel (without
+// room for them they are formed here).
+// n = 5,000 / 500 trees / 1.1e8 weighted updates: 1.32 ms (20.0 ms with one CTA
+// per row and window, a barrier and a chain of dependent loads per tree;
+// 1.6 ms with elements of several ranges taken together and conflicts resolved
+// by match.any, which serialises distinct values; 2.9 ms with elements staged
+// for the four warps of a CTA).
+template <int MODE, bool PRE>
+__global__ void __launch_bounds__(32)
+weighted_row_kernel(WRange* __restrict__ tab, int i0, const int32_t* __restrict__ memb,
+                    const double* __restrict__ wm, const int32_t* __restrict__ nin, const int32_t* __restrict__ nout,
+                    int n, int T, int win, double* __restrict__ out) {
+    extern __shared__ double2 wr_acc[];  // per column: x = accA, y = accB
+    const int i = i0 + blockIdx.x;
+    const int lane = threadIdx.x;
+    double* acc = reinterpret_cast<double*>(wr_acc);
+    int4* row = reinterpret_cast<int4*>(tab + (size_t)blockIdx.x * T);
     const int64_t rowoff = (int64_t)i * n - ((int64_t)i * (i - 1)) / 2 - i;  // + j gives [i][j]
     const int sI = nout[i] / 2;  // trees where i is OOB
     const double invI = sI > 0 ? __ddiv_rn(1.0, (double)sI) : 0.0;
-    for (int j = max(c0, i) + tid; j < c1; j += WR_THREADS) {
-        double v;
-        if (j == i) {
-            v = MODE == WR_RFGAP ? (sI == 0 ? 1.0 : 0.0) : 0.0;
-        } else if (MODE == WR_RFGAP) {
-            const int sJ = nout[j] / 2;
-            const double a = sI > 0 ? __dmul_rn(accA[j - c0], invI) : accA[j - c0];
-            const double bj = sJ > 0 ? __dmul_rn(accB[j - c0], __ddiv_rn(1.0, (double)sJ)) : accB[j - c0];
-            v = __ddiv_rn(__dadd_rn(a, bj), 2.0);
-        } else {
-            v = __dadd_rn(accA[j - c0], accB[j - c0]);
+    for (int c0 = i; c0 < n; c0 += win) {
+        const int c1 = min(n, c0 + win);
+        const bool last = c1 == n;
+        for (int k = lane; k < c1 - c0; k += 32) wr_acc[k] = make_double2(0.0, 0.0);
+        __syncwarp();
+        int4 nxt = lane < T ? row[lane] : make_int4(0, 0, 0, 0);
+        for (int tb = 0; tb < T; tb += 32) {
+            const int t = tb + lane;
+            const int4 raw = nxt;
+            if (tb + 32 < T) nxt = t + 32 < T ? row[t + 32] : make_int4(0, 0, 0, 0);
+            int lo = raw.x, len = raw.y & 0x7fffffff;
+            const int side = (unsigned)raw.y >> 31;
+            const int j0 = len > 0 ? __ldg(memb + (size_t)t * n + lo) : n;
+            unsigned todo = __ballot_sync(0xffffffffu, j0 < c1);
+            if (!todo) continue;
+            struct Batch {
+                int c[WR_BATCH], cnt[WR_BATCH], j[WR_BATCH];
+                double v[WR_BATCH];
+            };
+            auto fetch = [&](int c, int at, int sd, double wc, int& j, double& v) {
+                const size_t q = (size_t)(tb + c) * n + at;
+                j = __ldg(memb + q);
+                v = wc;
+                if (MODE != WR_PLAIN && !sd) {
+                    if (PRE) {
+                        v = __ldg(wm + q);
+                    } else {
+                        const double cj = (double)__ldg(nin + (size_t)(tb + c) * n + j);
+                        v = MODE == WR_RFGAP ? __dmul_rn(cj, wc) : __ddiv_rn(cj, wc);
+                    }
+                }
+            };
+            auto take = [&](Batch& b) {
+#pragma unroll
+                for (int u = 0; u < WR_BATCH; ++u) {
+                    const int c = todo ? __ffs(todo) - 1 : 0;
+                    b.c[u] = c;
+                    b.cnt[u] = todo ? __shfl_sync(0xffffffffu, len, c) : 0;
+                    const int at = __shfl_sync(0xffffffffu, lo, c), sd = __shfl_sync(0xffffffffu, side, c);
+                    const double wc = __hiloint2double(__shfl_sync(0xffffffffu, raw.w, c),
+                                                       __shfl_sync(0xffffffffu, raw.z, c));
+                    todo &= todo - 1;
+                    b.j[u] = n;
+                    b.v[u] = 0.0;
+                    if (lane < b.cnt[u]) fetch(c, at + lane, sd, wc, b.j[u], b.v[u]);
+                }
+            };
+            Batch cur;
+            take(cur);
+            while (cur.cnt[0] > 0) {
+                Batch ahead;
+                take(ahead);
+#pragma unroll
+                for (int u = 0; u < WR_BATCH; ++u) {
+                    if (cur.cnt[u] == 0) break;
+                    const int c = cur.c[u];
+                    const int sd = __shfl_sync(0xffffffffu, side, c);
+                    const bool in = cur.j[u] < c1;
+                    double* a = acc + sd - 2 * c0;
+                    if (in) a[2 * cur.j[u]] = __dadd_rn(a[2 * cur.j[u]], cur.v[u]);
+                    int used = __popc(__ballot_sync(0xffffffffu, in));
+                    if (used == 32 && cur.cnt[u] > 32) {  // the rest of a long range
+                        const int at = __shfl_sync(0xffffffffu, lo, c);
+                        const double wc = __hiloint2double(__shfl_sync(0xffffffffu, raw.w, c),
+                                                           __shfl_sync(0xffffffffu, raw.z, c));
+                        for (int off = 32;; off += 64) {
+                            int j1 = n, j2 = n;
+                            double v1 = 0.0, v2 = 0.0;
+                            if (off + lane < cur.cnt[u]) fetch(c, at + off + lane, sd, wc, j1, v1);
+                            if (off + 32 + lane < cur.cnt[u]) fetch(c, at + off + 32 + lane, sd, wc, j2, v2);
+                            if (j1 < c1) a[2 * j1] = __dadd_rn(a[2 * j1], v1);
+                            if (j2 < c1) a[2 * j2] = __dadd_rn(a[2 * j2], v2);
+                            const int got = __popc(__ballot_sync(0xffffffffu, j1 < c1)) +
+                                            __popc(__ballot_sync(0xffffffffu, j2 < c1));
+                            used += got;
+                            if (got < 64) break;
+                        }
+                    }
+                    if (lane == c) {
+                        lo += used;
+                        len -= used;
+                    }
+                    __syncwarp();  // this tree's adds come before the next one's
+                }
+                cur = ahead;
+            }
+            // the ranges go on from here in the next window
+            if (!last && t < T && lo != raw.x)
+                *reinterpret_cast<int2*>(row + t) = make_int2(lo, len | (raw.y & (int)WR_INBAG));
         }
-        out[rowoff + j] = v;
+        for (int j = c0 + lane; j < c1; j += 32) {
+            double v;
+            if (j == i) {
+                v = MODE == WR_RFGAP ? (sI == 0 ? 1.0 : 0.0) : 0.0;
+            } else {
+                const double2 ab = wr_acc[j - c0];
+                if (MODE == WR_RFGAP) {
+                    const int sJ = nout[j] / 2;
+                    const double a = sI > 0 ? __dmul_rn(ab.x, invI) : ab.x;
+                    const double bj = sJ > 0 ? __dmul_rn(ab.y, __ddiv_rn(1.0, (double)sJ)) : ab.y;
+                    v = __ddiv_rn(__dadd_rn(a, bj), 2.0);
+                } else {
+                    v = __dadd_rn(ab.x, ab.y);
+                }
+            }
+            out[rowoff + j] = v;
+        }
+        __syncwarp();  // the sums are cleared for the next window
     }
 }
 
@@ -423,6 +557,50 @@ rfx_status launch_casewise_votes(Ctx* c, const int32_t* d_leafnode, float* d_q) 
     return RFX_OK;
 }
 
+template <int MODE>
+static rfx_status weighted_rows(Ctx* c, const int32_t* key, const int64_t* segbase, const int32_t* segoff,
+                                const int32_t* memb, const long long* mass, double* out) {
+    const int n = c->n, T = c->T;
+    // the range table holds as many rows as WR_TABLE bytes take (all rows of
+    // the sizes whose matrix fits easily), fewer where memory is short
+    constexpr size_t WR_TABLE = (size_t)256 << 20;
+    Scratch sc(c);
+    const size_t row_bytes = sizeof(WRange) * (size_t)T;
+    int rows = (int)std::min<size_t>((size_t)n, std::max<size_t>(32, WR_TABLE / row_bytes));
+    WRange* tab = sc.get<WRange>((size_t)rows * T);
+    while (!tab && rows > 1) {
+        rows = (rows + 1) / 2;
+        tab = sc.get<WRange>((size_t)rows * T);
+    }
+    if (!tab) {
+        set_error("weighted pair sums: scratch allocation failed");
+        return RFX_ERR_OOM;
+    }
+    double* wm = MODE == WR_PLAIN ? nullptr : sc.get<double>((size_t)n * T);
+    if (wm) {
+        member_weight_kernel<MODE><<<dim3((n + 255) / 256, T), 256, 0, c->stream>>>(key, segbase, segoff, memb, mass,
+                                                                                    c->d_nin, n, wm);
+        RFX_CUDA(cudaGetLastError());
+        c->launches += 1;
+    }
+    const int win = std::min(WR_WINDOW, n);
+    const size_t smem = (size_t)win * sizeof(double2);
+    for (int i0 = 0; i0 < n; i0 += rows) {
+        const int i1 = std::min(n, i0 + rows);
+        weighted_ranges_kernel<MODE><<<dim3((i1 - i0 + 31) / 32, (T + 31) / 32), 256, 0, c->stream>>>(
+            key, segbase, segoff, memb, mass, c->d_nin, n, T, i0, i1, tab);
+        if (wm || MODE == WR_PLAIN)
+            weighted_row_kernel<MODE, true><<<i1 - i0, 32, smem, c->stream>>>(tab, i0, memb, wm, c->d_nin, c->d_nout,
+                                                                              n, T, win, out);
+        else
+            weighted_row_kernel<MODE, false><<<i1 - i0, 32, smem, c->stream>>>(tab, i0, memb, wm, c->d_nin, c->d_nout,
+                                                                               n, T, win, out);
+        RFX_CUDA(cudaGetLastError());
+        c->launches += 2;
+    }
+    return RFX_OK;
+}
+
 // Weighted FP64 pair sums (mode 0 case-wise, 2 unweighted) or the RF-GAP
 // matrix (mode 1), packed upper triangle, from leaf lists of keys `key`
 // (segbase/segoff/memb of those keys).
@@ -434,27 +612,12 @@ rfx_status launch_weighted_rows(Ctx* c, int mode, const int32_t* key, const int6
         set_error("weighted pair sums: scratch allocation failed");
         return RFX_ERR_OOM;
     }
-    key_mass_kernel<<<c->T, 128, 0, c->stream>>>(segbase, segoff, memb, c->d_nin, c->n, mass);
-    dim3 g(c->n, (c->n + WR_WINDOW - 1) / WR_WINDOW);
-    const size_t smem = 2 * (size_t)WR_WINDOW * sizeof(double);
-    RFX_CUDA(cudaFuncSetAttribute(weighted_row_kernel<WR_RFGAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    RFX_CUDA(cudaFuncSetAttribute(weighted_row_kernel<WR_CASEWISE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    RFX_CUDA(cudaFuncSetAttribute(weighted_row_kernel<WR_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    if (mode == WR_PLAIN)
-        weighted_row_kernel<WR_PLAIN><<<g, WR_THREADS, smem, c->stream>>>(key, segbase, segoff, memb, mass, c->d_nin,
-                                                                          c->d_nout, c->n, c->T, out);
-    else if (mode == WR_RFGAP)
-        weighted_row_kernel<WR_RFGAP><<<g, WR_THREADS, smem, c->stream>>>(key, segbase, segoff, memb, mass, c->d_nin,
-                                                                          c->d_nout, c->n, c->T, out);
-    else
-        weighted_row_kernel<WR_CASEWISE><<<g, WR_THREADS, smem, c->stream>>>(key, segbase, segoff, memb, mass,
-                                                                             c->d_nin, c->d_nout, c->n, c->T, out);
+    key_mass_kernel<<<c->T, 512, 0, c->stream>>>(segbase, segoff, memb, c->d_nin, c->n, mass);
     RFX_CUDA(cudaGetLastError());
-    c->launches += 2;
-    return RFX_OK;
+    c->launches += 1;
+    if (mode == WR_PLAIN) return weighted_rows<WR_PLAIN>(c, key, segbase, segoff, memb, mass, out);
+    if (mode == WR_RFGAP) return weighted_rows<WR_RFGAP>(c, key, segbase, segoff, memb, mass, out);
+    return weighted_rows<WR_CASEWISE>(c, key, segbase, segoff, memb, mass, out);
 }
 
 rfx_status launch_gap_keys(Ctx* c, const int32_t* d_leafnode, int32_t* d_key) {
