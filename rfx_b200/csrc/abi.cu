@@ -660,9 +660,9 @@ rfx_status rfx_route_oob(rfx_ctx* ctx, int32_t* q, int32_t* nout, int32_t* leaf)
             if ((st = copy_out(c, leaf, dleaf, sizeof(int32_t) * (size_t)c->T * c->n))) return st;
             any_host = true;
         }
-        // nout is produced by launch_route; run it as well (cheap)
+    } else if ((st = launch_route(c))) {
+        return st;
     }
-    if ((st = launch_route(c))) return st;
     c->routed = true;
     c->csr_built = false;
     if (q) {
@@ -775,7 +775,6 @@ static rfx_status casewise_votes_into(Ctx* c, float* dq) {
         return RFX_ERR_OOM;
     }
     rfx_status st = launch_route_leaf(c, dleaf);  // node ids, and nout
-    if (st == RFX_OK) st = launch_route(c);
     if (st == RFX_OK) {
         c->routed = true;
         c->csr_built = false;
@@ -898,7 +897,6 @@ rfx_status rfx_proximity_rfgap(rfx_ctx* ctx, double* P, size_t len) {
         }
         RFX_CUDA(cudaMemcpyAsync(dsb, sb.data(), sizeof(int64_t) * (T + 1), cudaMemcpyHostToDevice, c->stream));
         rfx_status s = launch_route_leaf(c, leaf);  // node ids (and nout)
-        if (s == RFX_OK) s = launch_route(c);
         if (s != RFX_OK) return s;
         c->routed = true;
         c->csr_built = false;
