@@ -9,8 +9,8 @@
 // Stage 1 (build_csr_kernel, one CTA per tree): a stable counting sort of the
 //   tree's samples by key = 2*leaf + inbag.  seg[t][k] .. seg[t][k+1] is the
 //   member range of key k in memb[t*n ...], members ascending by sample id.
-//   The CTA counts and scans the keys; a single warp then places the samples
-//   in index order, so equal keys keep index order.
+//   The CTA counts and scans the keys, then places the samples in index order,
+//   so equal keys keep index order.
 // Stage 2, row-owner: one CTA owns row i of S; for every tree it takes, in the
 //   member list of the opposite bag status of i's leaf, the members j > i and
 //   adds 1 to a shared-memory counter per member; the accumulated row is then
@@ -33,8 +33,12 @@ namespace {
 // ---------------------------------------------------------------------------
 // Stage 1
 // ---------------------------------------------------------------------------
-constexpr int CSR_THREADS = 128;
-constexpr int CSR_PREFETCH = 16;  // 32-sample groups loaded ahead by the scattering warp
+constexpr int CSR_THREADS = 256;
+constexpr int CSR_WARPS = CSR_THREADS / 32;
+constexpr int CSR_MINB = 4;     // CTAs per SM: more trees at once scatter past L2 (0.30 ms; 5: 0.31)
+constexpr int CSR_GROUPS = 8;   // 32-sample groups per warp and turn of the scatter
+constexpr int CSR_TAGS = 512;   // tag bytes per warp
+constexpr int CSR_COUNT = 8;    // keys in flight per thread of the histogram
 
 // Key counters of the CSR build: in shared memory as CT (16-bit when every
 // count and offset stays below 65536, so twice as many trees fit per SM), or
@@ -49,24 +53,42 @@ struct CsrCounters {
         if (sm) s[k] = (CT)v;
         else g[k] = v;
     }
-    __device__ __forceinline__ void inc(int k) {
-        if (!sm) atomicAdd(g + k, 1);
-        else if (sizeof(CT) == 2) atomicAdd(reinterpret_cast<unsigned int*>(s) + (k >> 1), 1u << ((k & 1) << 4));
-        else atomicAdd(reinterpret_cast<int*>(s) + k, 1);
+    __device__ __forceinline__ void add(int k, int v) {
+        if (!sm) atomicAdd(g + k, v);
+        else if (sizeof(CT) == 4) atomicAdd(reinterpret_cast<int*>(s) + k, v);
+        else atomicAdd(reinterpret_cast<unsigned int*>(s) + (k >> 1), (unsigned)v << ((k & 1) << 4));
     }
 };
 
+// Turns between the warps of a CTA: warp w waits at named barrier 1 + w, where
+// the warp before it arrives (64 threads: 32 wait, 32 arrive); shared-memory
+// writes before the arrival are visible after the wait.
+__device__ __forceinline__ void csr_turn_wait(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void csr_turn_pass(int id) {
+    __threadfence_block();
+    asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
+
 // One CTA per tree.  All warps build the key histogram; the exclusive scan
-// runs over four quarters in parallel; warp 0 alone then scatters the samples
-// in index order (equal keys inside a 32-sample group are ranked by lane), so
-// every key's member list is ascending by sample id.
-template <typename CT>
-__global__ void __launch_bounds__(CSR_THREADS)
+// runs over one part per warp in parallel; then the samples are scattered in
+// index order, so every key's member list is ascending by sample id.  What
+// must be ordered there is only the step of the key counters: the warps take
+// CSR_GROUPS groups of 32 samples each, find the lanes of equal keys, and step
+// the counters in turn, handed from warp to warp by named barriers; the member
+// stores follow outside the turn.  SM: every tree's counters are in shared
+// memory (no test per access, which the chain of counter steps would pay for).
+// n = 50,000 / 1,000 trees: 0.30 ms (0.68 ms with one warp per tree doing all
+// of it, the same at 300 trees: its chain of about 750 cycles a group was the
+// bound; match.any or a ballot per key bit for the equal lanes cost more than
+// the tags).
+template <typename CT, bool SM>
+__global__ void __launch_bounds__(CSR_THREADS, CSR_MINB)
 build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restrict__ segbase,
                  int32_t* __restrict__ segoff, int32_t* __restrict__ memb, int smem_keys,
                  uint32_t* __restrict__ err) {
     extern __shared__ int32_t cnt[];
-    __shared__ int qtot[CSR_THREADS / 32];
+    __shared__ int qtot[CSR_WARPS];
+    __shared__ uint8_t s_tag[CSR_WARPS][CSR_TAGS];
     const int t = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int64_t sb = segbase[t];
@@ -76,7 +98,7 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
     int32_t* so = segoff + sb;
     // counters: shared memory when the key table fits, else the tree's own
     // segment-offset table in global memory (slower, still exact)
-    const bool use_smem = K + 1 <= smem_keys;
+    const bool use_smem = SM || K + 1 <= smem_keys;
     CsrCounters<CT> ctr{reinterpret_cast<CT*>(cnt), so, use_smem};
     for (int k = tid; k <= K; k += CSR_THREADS) ctr.set(k, 0);
     if (use_smem && sizeof(CT) == 2 && tid == 0) ctr.s[K + 1] = 0;  // the other half of the last counter word
@@ -84,13 +106,24 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
     // samples without a terminal node (key -1) go to the slot after the
     // last key, so they follow every key's members (segoff[K] still marks
     // the end of the keyed members)
-    for (int i = tid; i < n; i += CSR_THREADS) {
-        const int k = __ldg(kt + i);
-        ctr.inc(k >= 0 ? k : K);
+    int none = 0;  // counted in a register: half the samples can share that slot
+    for (int i0 = tid; i0 < n; i0 += CSR_THREADS * CSR_COUNT) {
+        int k[CSR_COUNT];
+#pragma unroll
+        for (int u = 0; u < CSR_COUNT; ++u) {
+            const int i = i0 + u * CSR_THREADS;
+            k[u] = i < n ? __ldg(kt + i) : -2;
+        }
+#pragma unroll
+        for (int u = 0; u < CSR_COUNT; ++u)
+            if (k[u] >= 0) ctr.add(k[u], 1);
+            else none += k[u] == -1;
     }
+    none = __reduce_add_sync(0xffffffffu, none);
+    if (lane == 0 && none) ctr.add(K, none);
     __syncthreads();
-    // exclusive scan of K+1 counters: quarter q = [q*Q, min((q+1)*Q, K+1))
-    const int Q = (K + 1 + 3) / 4;
+    // exclusive scan of K+1 counters: part q = [q*Q, min((q+1)*Q, K+1))
+    const int Q = (K + CSR_WARPS) / CSR_WARPS;
     const int q0 = w * Q, q1 = min(K + 1, q0 + Q);
     int carry = 0;
     for (int k0 = q0; k0 < q1; k0 += 32) {
@@ -115,43 +148,57 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
         if (use_smem) so[k] = v;
     }
     __syncthreads();
-    if (w != 0) return;
-    // stable scatter by one warp, samples in index order; the next batch of
-    // keys is loaded while the current one is placed
-    int kv[CSR_PREFETCH], kn[CSR_PREFETCH];
-    // slot per sample: its key, K for key -1, -1 past the end
+    // stable scatter: batch r * CSR_WARPS + w of 32 * CSR_GROUPS samples is
+    // warp w's in round r
+    const unsigned below = (1u << lane) - 1u;
+    volatile uint8_t* tag = s_tag[w];
+    constexpr int BATCH = 32 * CSR_GROUPS;
+    const int rounds = (n + BATCH * CSR_WARPS - 1) / (BATCH * CSR_WARPS);
+    for (int rd = 0; rd < rounds; ++rd) {
+        const int base = (rd * CSR_WARPS + w) * BATCH;
+        // slot per sample: its key, K for key -1, K + 1 past the end
+        int kv[CSR_GROUPS];
 #pragma unroll
-    for (int u = 0; u < CSR_PREFETCH; ++u) {
-        const int i = u * 32 + lane;
-        const int k = i < n ? __ldg(kt + i) : 0;
-        kv[u] = i < n ? (k >= 0 ? k : K) : -1;
-    }
-    for (int base = 0; base < n; base += 32 * CSR_PREFETCH) {
-        const int nb = base + 32 * CSR_PREFETCH;
-#pragma unroll
-        for (int u = 0; u < CSR_PREFETCH; ++u) {
-            const int i = nb + u * 32 + lane;
-            const int k = i < n ? __ldg(kt + i) : 0;
-            kn[u] = i < n ? (k >= 0 ? k : K) : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < CSR_PREFETCH; ++u) {
+        for (int u = 0; u < CSR_GROUPS; ++u) {
             const int i = base + u * 32 + lane;
+            const int k = i < n ? __ldg(kt + i) : 0;
+            kv[u] = i < n ? (k >= 0 ? k : K) : K + 1;
+        }
+        // grp: the lanes of the same slot.  Every lane writes its number into a
+        // tag byte picked by its slot's low bits; a lane that reads another's
+        // shares its slot (or only the tag) with someone, and the distinct
+        // slots of those lanes are gone through by ballots
+        unsigned grp[CSR_GROUPS];
+#pragma unroll
+        for (int u = 0; u < CSR_GROUPS; ++u) {
             const int k = kv[u];
-            const unsigned grp = __match_any_sync(0xffffffffu, k);
-            const int leader = __ffs(grp) - 1;
-            const int rank = __popc(grp & ((1u << lane) - 1u));
-            int start = 0;
-            if (k >= 0 && lane == leader) {
-                start = ctr.get(k);
-                ctr.set(k, start + __popc(grp));
+            grp[u] = 1u << lane;
+            if (base + u * 32 >= n) continue;
+            tag[k & (CSR_TAGS - 1)] = (uint8_t)lane;
+            __syncwarp();
+            unsigned lost = __ballot_sync(0xffffffffu, tag[k & (CSR_TAGS - 1)] != lane);
+            while (lost) {
+                const int kk = __shfl_sync(0xffffffffu, k, __ffs(lost) - 1);
+                const unsigned g = __ballot_sync(0xffffffffu, k == kk);
+                if (k == kk) grp[u] = g;
+                lost &= ~g;
             }
-            start = __shfl_sync(0xffffffffu, start, leader);
-            if (k >= 0) mt[start + rank] = i;
             __syncwarp();
         }
+        // turn: after the warp before (and, for warp 0, the last warp of the round before)
+        if (w > 0 || rd > 0) csr_turn_wait(1 + w);
+        int start[CSR_GROUPS];
 #pragma unroll
-        for (int u = 0; u < CSR_PREFETCH; ++u) kv[u] = kn[u];
+        for (int u = 0; u < CSR_GROUPS; ++u) {
+            start[u] = kv[u] <= K ? ctr.get(kv[u]) : 0;
+            __syncwarp();
+            if (kv[u] <= K && (grp[u] >> lane) == 1u) ctr.set(kv[u], start[u] + __popc(grp[u]));  // the slot's last lane
+            __syncwarp();
+        }
+        if (w + 1 < CSR_WARPS || rd + 1 < rounds) csr_turn_pass(w + 1 < CSR_WARPS ? 2 + w : 1);
+#pragma unroll
+        for (int u = 0; u < CSR_GROUPS; ++u)
+            if (kv[u] <= K) mt[start[u] + __popc(grp[u] & below)] = base + u * 32 + lane;
     }
     // global-counter path: the counters now hold segment ends; a follow-up
     // kernel (fix_global_segoff_kernel) turns them back into starts
@@ -1144,23 +1191,34 @@ finishprox_kernel(const TS* __restrict__ S, const double* __restrict__ inv, int 
 
 }  // namespace
 
+// The leaf-list kernel: with every tree's counters in shared memory (tables of
+// up to smem_keys keys), or with the larger tables' counters in global memory
+// and the pass that turns their ends back into starts.
+template <typename CT>
+static rfx_status csr_launch(cudaStream_t s, int dev_smem, const int32_t* key, int n, int T, const int64_t* segbase,
+                             int32_t* segoff, int32_t* memb, int max_keys, int smem_keys, size_t smem, uint32_t* err) {
+    const bool fits = max_keys + 1 <= smem_keys;
+    auto kernel = fits ? build_csr_kernel<CT, true> : build_csr_kernel<CT, false>;
+    if (rfx_status s0 = allow_dyn_smem(kernel, dev_smem)) return s0;
+    kernel<<<T, CSR_THREADS, smem, s>>>(key, n, segbase, segoff, memb, smem_keys, err);
+    RFX_CUDA(cudaGetLastError());
+    if (!fits) {
+        fix_global_segoff_kernel<<<T, 32, 0, s>>>(segbase, segoff, smem_keys);
+        RFX_CUDA(cudaGetLastError());
+    }
+    return RFX_OK;
+}
+
 // Leaf lists of arbitrary keys (key per (tree, sample) in [0, K_t), or -1),
 // for callers with their own key tables (RF-GAP's node-id keys).
 rfx_status launch_build_csr_raw(cudaStream_t s, int device, const int32_t* key, int n, int T, const int64_t* segbase,
                                 int32_t* segoff, int32_t* memb, int max_keys, uint32_t* err) {
     int dev_smem = 0;
     RFX_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    int smem_keys = std::min(max_keys + 1, (dev_smem - 1024) / 4);
+    int smem_keys = std::min(max_keys + 1, (dev_smem - 6144) / 4);
     smem_keys = std::max(smem_keys, 32);
     const size_t smem = (size_t)smem_keys * sizeof(int32_t);
-    if (rfx_status s0 = allow_dyn_smem(build_csr_kernel<int32_t>, dev_smem)) return s0;
-    build_csr_kernel<int32_t><<<T, CSR_THREADS, smem, s>>>(key, n, segbase, segoff, memb, smem_keys, err);
-    RFX_CUDA(cudaGetLastError());
-    if (max_keys + 1 > smem_keys) {
-        fix_global_segoff_kernel<<<T, 32, 0, s>>>(segbase, segoff, smem_keys);
-        RFX_CUDA(cudaGetLastError());
-    }
-    return RFX_OK;
+    return csr_launch<int32_t>(s, dev_smem, key, n, T, segbase, segoff, memb, max_keys, smem_keys, smem, err);
 }
 
 rfx_status launch_build_csr(Ctx* c) {
@@ -1169,21 +1227,14 @@ rfx_status launch_build_csr(Ctx* c) {
     // budget per tree-warp; several warps (trees) share an SM
     const bool narrow = c->n < 65536;  // counts and offsets fit 16 bits
     const int csz = narrow ? 2 : 4;
-    int smem_keys = std::min(c->max_keys + 1, (dev_smem - 1024) / csz - 2);
+    int smem_keys = std::min(c->max_keys + 1, (dev_smem - 6144) / csz - 2);
     smem_keys = std::max(smem_keys, 32);
     const size_t smem = ((size_t)(smem_keys + 2) * csz + 3) & ~(size_t)3;
     StageTimer st(c, ST_CSR, c->max_keys + 1 > smem_keys ? 2 : 1);
-    if (rfx_status s0 = allow_dyn_smem(build_csr_kernel<uint16_t>, dev_smem)) return s0;
-    if (rfx_status s0 = allow_dyn_smem(build_csr_kernel<int32_t>, dev_smem)) return s0;
-    (narrow ? build_csr_kernel<uint16_t> : build_csr_kernel<int32_t>)<<<c->T, CSR_THREADS, smem, c->stream>>>(
-        c->d_key, c->n, c->d_segbase, c->d_segoff, c->d_memb, smem_keys,
-                                                    c->d_err);
-    RFX_CUDA(cudaGetLastError());
-    if (c->max_keys + 1 > smem_keys) {
-        fix_global_segoff_kernel<<<c->T, 32, 0, c->stream>>>(c->d_segbase, c->d_segoff, smem_keys);
-        RFX_CUDA(cudaGetLastError());
-    }
-    return RFX_OK;
+    return narrow ? csr_launch<uint16_t>(c->stream, dev_smem, c->d_key, c->n, c->T, c->d_segbase, c->d_segoff,
+                                         c->d_memb, c->max_keys, smem_keys, smem, c->d_err)
+                  : csr_launch<int32_t>(c->stream, dev_smem, c->d_key, c->n, c->T, c->d_segbase, c->d_segoff,
+                                        c->d_memb, c->max_keys, smem_keys, smem, c->d_err);
 }
 
 int pairs_window(const Ctx* c) {
@@ -1344,17 +1395,12 @@ rfx_status launch_pairs_pipeline_raw(const PairsRawArgs& a, cudaStream_t stream)
     RFX_CUDA(cudaGetDevice(&dev));
     RFX_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const int max_keys = 2 * a.max_leaves;
-    int smem_keys = std::min(max_keys + 1, (dev_smem - 1024) / 4);
+    int smem_keys = std::min(max_keys + 1, (dev_smem - 6144) / 4);
     smem_keys = std::max(smem_keys, 32);
     const size_t smem = (size_t)smem_keys * sizeof(int32_t);
-    if (rfx_status s0 = allow_dyn_smem(build_csr_kernel<int32_t>, dev_smem)) return s0;
-    build_csr_kernel<int32_t><<<a.T, CSR_THREADS, smem, stream>>>(a.key, a.n, a.segbase, a.segoff, a.memb, smem_keys,
-                                                         a.err);
-    RFX_CUDA(cudaGetLastError());
-    if (max_keys + 1 > smem_keys) {
-        fix_global_segoff_kernel<<<a.T, 32, 0, stream>>>(a.segbase, a.segoff, smem_keys);
-        RFX_CUDA(cudaGetLastError());
-    }
+    if (rfx_status s0 = csr_launch<int32_t>(stream, dev_smem, a.key, a.n, a.T, a.segbase, a.segoff, a.memb, max_keys,
+                                            smem_keys, smem, a.err))
+        return s0;
     dim3 g((a.n + OPP_TILE - 1) / OPP_TILE, (a.T + OPP_TILE - 1) / OPP_TILE);
     opp_kernel<<<g, OPP_TILE * 8, 0, stream>>>(a.key, a.segoff, a.segbase, a.memb, a.n, a.T, nullptr, a.opp);
     RFX_CUDA(cudaGetLastError());
