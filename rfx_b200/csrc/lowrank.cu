@@ -630,23 +630,19 @@ __global__ void gram_sum_w_kernel(const double* __restrict__ part, int nparts, i
     const int e = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (e >= cnt) return;
-    double v = 0.0;
-    for (int q = lane; q < nparts; q += 32) v += part[(size_t)q * cnt + e];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    const double v = warp_part_sum(part + e, nparts, (size_t)cnt, lane);
     if (lane == 0) G[e] = v;
 }
 
 // One CTA: T = L^{-T} for G = L L^T (w x w), in shared memory (dynamic).
-__global__ void chol_inv_w_kernel(const double* __restrict__ G, int w, double* __restrict__ Tm, int* __restrict__ bad) {
+__global__ void __launch_bounds__(1024) chol_inv_w_kernel(const double* __restrict__ G, int w, double* __restrict__ Tm, int* __restrict__ bad) {
     extern __shared__ double sm[];
     double* L = sm;
     double* Li = sm + w * w;
     __shared__ double flag;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) L[e] = G[e];
     __syncthreads();
-    if (!cta_cholesky(L, w, w, &flag) && threadIdx.x == 0) *bad = 1;
-    cta_tri_inverse(L, Li, w, w);
+    if (!cta_cholesky_inverse(L, Li, w, w, &flag) && threadIdx.x == 0) *bad = 1;
     for (int e = threadIdx.x; e < w * w; e += blockDim.x) {
         const int i = e / w, j = e % w;
         Tm[i * w + j] = Li[j * w + i];
@@ -1031,7 +1027,7 @@ rfx_status lowrank_compute(Ctx* c, int k, int oversample, int power_iters, int p
         float* tmp = Z;
         for (int pass = 0; pass < 2; ++pass) {
             gram(cur, cur);
-            chol_inv_w_kernel<<<1, 256, sm2, s>>>(Gm, w, Tm, bad);
+            chol_inv_w_kernel<<<1, 1024, sm2, s>>>(Gm, w, Tm, bad);
             float* dst = pass == 0 ? tmp : out;
             right_mul_kernel<<<(n + RM_ROWS - 1) / RM_ROWS, right_mul_threads(w), right_mul_smem(w, w), s>>>(
                 cur, Tm, n, w, w, dst);

@@ -122,7 +122,7 @@ __global__ void mds_b_kernel(const float* __restrict__ P, const int32_t* __restr
 // contiguous bulk copy that lands in a layout whose fragment reads are free
 // of bank conflicts.  A CTA of four warps owns 64 rows and one range of
 // kchunk columns; each 64-column step brings the B tile and the matching
-// 64 x 16 block of V (pre-arranged in fragment order by bv_pack_kernel)
+// 64 x 16 block of V (in fragment order, written so by the kernels that make V)
 // through a DB_STAGES-deep mbarrier pipeline, two bulk copies per step.  Warp w multiplies rows 16w..16w+15 by both 8-column halves of V.
 // The partial products go to Wpart[range] and are added in range order.
 constexpr int GT = 64;
@@ -177,15 +177,11 @@ __device__ __forceinline__ void dmma(double* c, double a0, double a1, double b) 
                  : "d"(a0), "d"(a1), "d"(b));
 }
 
-// Vf = V in fragment order, npad rows (rows >= n zero): within each 4-row
-// step, element (k, c) sits at (c / 8) * 32 + (c % 8) * 4 + k % 4, so the
-// lanes of a warp read 32 consecutive doubles per fragment.
-__global__ void bv_pack_kernel(const double* __restrict__ V, int n, int npad, double* __restrict__ Vf) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)npad * S_BLK) return;
-    const int k = (int)(idx / S_BLK), c = (int)(idx % S_BLK);
-    const size_t dst = (size_t)(k >> 2) * 64 + (c >> 3) * 32 + (c & 7) * 4 + (k & 3);
-    Vf[dst] = k < n ? V[idx] : 0.0;
+// Position of element (k, c) of an n x S_BLK block in fragment order (the
+// lanes of a warp read 32 consecutive doubles per fragment): within each 4-row
+// step at (c / 8) * 32 + (c % 8) * 4 + k % 4.
+__device__ __forceinline__ size_t frag_pos(int k, int c) {
+    return (size_t)(k >> 2) * 64 + (c >> 3) * 32 + (c & 7) * 4 + (k & 3);
 }
 
 __global__ void __launch_bounds__(128, 1) dgemm_bv_kernel(const double* __restrict__ B, int nt,
@@ -310,49 +306,93 @@ __global__ void gram_sum_kernel(const double* __restrict__ part, int nparts, dou
     const int e = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (e >= S_BLK * S_BLK) return;
-    double v = 0.0;
-    for (int q = lane; q < nparts; q += 32) v += part[(size_t)q * (S_BLK * S_BLK) + e];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    const double v = warp_part_sum(part + e, nparts, S_BLK * S_BLK, lane);
     if (lane == 0) G[e] = v;
 }
 
+// Up to GRAM_FUSE partials (one load a lane) are added by the kernels below
+// themselves, in the same order, which saves the launch; more go through
+// gram_sum_kernel over the whole GPU first.
+constexpr int GRAM_FUSE = 32;
+constexpr int SMALL_THREADS = 512;
+
+// The 16 x 16 matrix into shared memory (leading dim ld): from G, or summed
+// from nparts <= GRAM_FUSE partials (a warp takes every 16th entry).
+__device__ __forceinline__ void load_gram(const double* __restrict__ G, const double* __restrict__ part, int nparts,
+                                          double* out, int ld) {
+    if (!part) {
+        for (int e = threadIdx.x; e < S_BLK * S_BLK; e += SMALL_THREADS) out[(e / S_BLK) * ld + e % S_BLK] = G[e];
+        return;
+    }
+    constexpr int NW = SMALL_THREADS / 32, PER = S_BLK * S_BLK / NW;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double v[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] = lane < nparts ? part[(size_t)lane * (S_BLK * S_BLK) + w + u * NW] : 0.0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) v[u] += __shfl_xor_sync(0xffffffffu, v[u], d);
+        const int e = w + u * NW;
+        if (lane == 0) out[(e / S_BLK) * ld + e % S_BLK] = v[u];
+    }
+}
+
 // One CTA: Cholesky of G and the inverse of its factor, T = L^{-T} (S x S).
-__global__ void chol_inv_kernel(const double* __restrict__ G, double* __restrict__ Tm, int* __restrict__ bad) {
+// A serial chain (16 square roots and divisions): 9.5 us from G, 15 us with
+// the sum of 32 partials (18 us, and 2 for the sum's own launch, with a dot
+// product per entry in one thread's chain).
+__global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* __restrict__ G,
+                                                                 const double* __restrict__ part, int nparts,
+                                                                 double* __restrict__ Tm, int* __restrict__ bad) {
     __shared__ double L[S_BLK * S_BLK], Li[S_BLK * S_BLK];
     __shared__ double flag;
-    for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) L[e] = G[e];
+    load_gram(G, part, nparts, L, S_BLK);
     __syncthreads();
-    if (!cta_cholesky(L, S_BLK, S_BLK, &flag) && threadIdx.x == 0) *bad = 1;
-    cta_tri_inverse(L, Li, S_BLK, S_BLK);
+    if (!cta_cholesky_inverse(L, Li, S_BLK, S_BLK, &flag) && threadIdx.x == 0) *bad = 1;
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) {
         const int i = e / S_BLK, j = e % S_BLK;
         Tm[i * S_BLK + j] = Li[j * S_BLK + i];  // (L^{-1})^T
     }
 }
 
-// V = W T (rows of W times an S x S matrix).
+// V = W T (rows of W times an S x S matrix), and with Vf the same in fragment
+// order for the next product.
 __global__ void dright_kernel(const double* __restrict__ W, const double* __restrict__ Tm, int n,
-                              double* __restrict__ V) {
+                              double* __restrict__ V, double* __restrict__ Vf) {
     __shared__ double Ts[S_BLK * S_BLK];
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) Ts[e] = Tm[e];
     __syncthreads();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (size_t)n * S_BLK) return;
     const int r = (int)(idx / S_BLK), c = (int)(idx % S_BLK);
+    double w[S_BLK];
+    const double2* wr = reinterpret_cast<const double2*>(W + (size_t)r * S_BLK);
+#pragma unroll
+    for (int k = 0; k < S_BLK / 2; ++k) {
+        const double2 x = __ldg(wr + k);
+        w[2 * k] = x.x;
+        w[2 * k + 1] = x.y;
+    }
     double v = 0.0;
-    for (int k = 0; k < S_BLK; ++k) v = fma(W[(size_t)r * S_BLK + k], Ts[k * S_BLK + c], v);
+#pragma unroll
+    for (int k = 0; k < S_BLK; ++k) v = fma(w[k], Ts[k * S_BLK + c], v);
     V[idx] = v;
+    if (Vf) Vf[frag_pos(r, c)] = v;
 }
 
 // One CTA: eigen-decomposition of the S x S projection H (symmetrised).
-__global__ void rr_kernel(const double* __restrict__ H, double* __restrict__ evals, double* __restrict__ evecs) {
+__global__ void __launch_bounds__(SMALL_THREADS) rr_kernel(const double* __restrict__ H,
+                                                           const double* __restrict__ part, int nparts,
+                                                           double* __restrict__ evals, double* __restrict__ evecs) {
     constexpr int LD = S_BLK + 1;
-    __shared__ double A[S_BLK * LD], U[S_BLK * LD];
+    __shared__ double Hs[S_BLK * S_BLK], A[S_BLK * LD], U[S_BLK * LD];
     __shared__ int pairs[2 * 64];
+    load_gram(H, part, nparts, Hs, S_BLK);
+    __syncthreads();
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) {
         const int i = e / S_BLK, j = e % S_BLK;
-        A[i * LD + j] = 0.5 * (H[i * S_BLK + j] + H[j * S_BLK + i]);
+        A[i * LD + j] = 0.5 * (Hs[i * S_BLK + j] + Hs[j * S_BLK + i]);
     }
     __syncthreads();
     cta_jacobi(A, U, S_BLK, LD, 30, pairs);
@@ -384,14 +424,21 @@ __device__ __forceinline__ uint64_t start_mix(uint64_t z) {
 }
 
 // out = a X + b Y + c Z over an n x S_BLK block (Z may be null); the
-// three-term recurrence of the Chebyshev filter.
-__global__ void block_axpby_kernel(double a, const double* __restrict__ X, double b, const double* __restrict__ Y,
-                                   double c, const double* __restrict__ Z, int64_t count, double* __restrict__ out) {
+// three-term recurrence of the Chebyshev filter.  X is the sum of ksn partial
+// products in range order (ksn = 1: a plain block); out is also written in
+// fragment order for the next product (Vf), so a filter step is two launches,
+// the product and this.
+__global__ void block_axpby_kernel(double a, const double* __restrict__ X, int ksn, double b,
+                                   const double* __restrict__ Y, double c, const double* __restrict__ Z,
+                                   int64_t count, double* __restrict__ out, double* __restrict__ Vf) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
-    double v = __dadd_rn(__dmul_rn(a, X[e]), __dmul_rn(b, Y[e]));
+    double x = X[e];
+    for (int s = 1; s < ksn; ++s) x += X[(size_t)s * count + e];
+    double v = __dadd_rn(__dmul_rn(a, x), __dmul_rn(b, Y[e]));
     if (Z) v = __dadd_rn(v, __dmul_rn(c, Z[e]));
     out[e] = v;
+    Vf[frag_pos((int)(e / S_BLK), (int)(e % S_BLK))] = v;
 }
 
 __global__ void start_block_kernel(double* __restrict__ V, int64_t count, uint64_t seed) {
@@ -406,11 +453,14 @@ __global__ void start_block_kernel(double* __restrict__ V, int64_t count, uint64
 // Subspace iteration on the symmetric operator applied by `apply` (W = B V),
 // returning the k largest eigenpairs above 1e-10: coordinates n x k in `out`
 // (device) and eigenvalues in `evals_out` (host).  Shared by the full-matrix
-// and the factor MDS.
+// and the factor MDS.  The full-matrix form (cheb > 0) keeps the block in
+// fragment order in Vf beside every write of V, and its `apply` leaves the
+// product as ksn partials in Wpart (W gets their sum when it is given).
 template <typename Apply>
 rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double* d_out, double* evals_out,
                          uint64_t seed, double tol = 1e-14, const double* warm_in = nullptr, double* keep_out = nullptr,
-                         int* iters_out = nullptr, bool floor_stop = false, int cheb = 0) {
+                         int* iters_out = nullptr, bool floor_stop = false, int cheb = 0, double* Vf = nullptr,
+                         const double* Wpart = nullptr, int ksn = 0) {
     cudaStream_t s = c->stream;
     Scratch d(c);
     double* V = d.get<double>((size_t)n * S_BLK);
@@ -449,20 +499,24 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
         set_error("MDS: device allocation failed");
         return RFX_ERR_OOM;
     }
+    // Gram matrix of X and Y: partials, and their sum in G unless the kernel
+    // that reads it adds the few there are
+    const double* fuse = gb <= GRAM_FUSE ? gpart : nullptr;
     auto gram = [&](const double* X, const double* Y) {
         dgram_kernel<<<gb, 256, 0, s>>>(X, Y, n, gpart);
-        gram_sum_kernel<<<S_BLK * S_BLK * 32 / 256, 256, 0, s>>>(gpart, gb, G);
+        if (!fuse) gram_sum_kernel<<<S_BLK * S_BLK * 32 / 256, 256, 0, s>>>(gpart, gb, G);
+        c->launches += fuse ? 1 : 2;
     };
     // CholeskyQR2: Out = (src L1^{-T}) L2^{-T}, through the temporary Xt
     auto orth = [&](const double* src, double* Out) -> rfx_status {
         const unsigned gr = (unsigned)(((size_t)n * S_BLK + 255) / 256);
         gram(src, src);
-        chol_inv_kernel<<<1, 128, 0, s>>>(G, Tm, bad);
-        dright_kernel<<<gr, 256, 0, s>>>(src, Tm, n, Xt);
+        chol_inv_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, Tm, bad);
+        dright_kernel<<<gr, 256, 0, s>>>(src, Tm, n, Xt, nullptr);
         gram(Xt, Xt);
-        chol_inv_kernel<<<1, 128, 0, s>>>(G, Tm, bad);
-        dright_kernel<<<gr, 256, 0, s>>>(Xt, Tm, n, Out);
-        c->launches += 8;
+        chol_inv_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, Tm, bad);
+        dright_kernel<<<gr, 256, 0, s>>>(Xt, Tm, n, Out, Vf);
+        c->launches += 4;
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
     };
@@ -474,8 +528,8 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
     // the k largest against the previous check into *delta
     auto ritz = [&](double* delta) -> rfx_status {
         gram(V, W);
-        rr_kernel<<<1, 128, 0, s>>>(G, ev, U);
-        c->launches += 3;
+        rr_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, ev, U);
+        c->launches += 1;
         RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
         RFX_CUDA(cudaStreamSynchronize(s));
         std::vector<double> a = cur, b = prev;
@@ -505,7 +559,7 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
             return RFX_ERR_OOM;
         }
         const int64_t cnt = (int64_t)n * S_BLK;
-        const unsigned gb = (unsigned)((cnt + 255) / 256);
+        const unsigned cb = (unsigned)((cnt + 255) / 256);
         for (int q = 0; q < 10; ++q) {
             if ((st = apply(V, W)) != RFX_OK) return st;
             if ((st = orth(W, V)) != RFX_OK) return st;
@@ -534,14 +588,17 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
             const double cc = 0.5 * (lo + hi), ee = 0.5 * (hi - lo);
             if (!(ee > 0.0)) break;
             // Y0 = V, Y1 = (B V - cc V) / ee, Y_{j+1} = 2 (B Y_j - cc Y_j) / ee - Y_{j-1}
-            RFX_CUDA(cudaMemcpyAsync(Y0, V, sizeof(double) * cnt, cudaMemcpyDeviceToDevice, s));
-            block_axpby_kernel<<<gb, 256, 0, s>>>(1.0 / ee, W, -cc / ee, V, 0.0, nullptr, cnt, Y1);
+            // (the first step reads V itself as Y0)
+            block_axpby_kernel<<<cb, 256, 0, s>>>(1.0 / ee, W, 1, -cc / ee, V, 0.0, nullptr, cnt, Y1, Vf);
             c->launches += 1;
+            const double* before = V;
             for (int j = 2; j <= cheb; ++j) {
-                if ((st = apply(Y1, W)) != RFX_OK) return st;
+                if ((st = apply(Y1, nullptr)) != RFX_OK) return st;
                 ++matvecs;
-                block_axpby_kernel<<<gb, 256, 0, s>>>(2.0 / ee, W, -2.0 * cc / ee, Y1, -1.0, Y0, cnt, Y2);
+                block_axpby_kernel<<<cb, 256, 0, s>>>(2.0 / ee, Wpart, ksn, -2.0 * cc / ee, Y1, -1.0, before, cnt, Y2,
+                                                      Vf);
                 c->launches += 1;
+                before = Y1;
                 std::swap(Y0, Y1);
                 std::swap(Y1, Y2);
             }
@@ -555,8 +612,8 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
         if (check) {
             // Rayleigh-Ritz on span(V): H = V^T (B V)
             gram(V, W);
-            rr_kernel<<<1, 128, 0, s>>>(G, ev, U);
-            c->launches += 3;
+            rr_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, ev, U);
+            c->launches += 1;
             RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
             RFX_CUDA(cudaStreamSynchronize(s));
             std::vector<double> a = cur, b = prev;
@@ -640,10 +697,7 @@ __global__ void part_sum_kernel(const TV* __restrict__ part, int nparts, int cnt
     const int e = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (e >= cnt) return;
-    TV s = 0;
-    for (int q = lane; q < nparts; q += 32) s += part[(size_t)q * cnt + e];
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    const TV s = warp_part_sum(part + e, nparts, (size_t)cnt, lane);
     if (lane == 0) out[e] = s * scale;
 }
 
@@ -1131,18 +1185,20 @@ rfx_status launch_mds3d_full(Ctx* c, const float* dP, double* d_coords, double* 
         return RFX_ERR_OOM;
     }
     RFX_CUDA(cudaFuncSetAttribute(dgemm_bv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DB_SMEM));
-    auto apply = [&](const double* V, double* W) -> rfx_status {
-        bv_pack_kernel<<<(unsigned)(((size_t)npad * S_BLK + 255) / 256), 256, 0, s>>>(V, n, npad, Vf);
+    // rows past n of the block in fragment order stay zero
+    RFX_CUDA(cudaMemsetAsync(Vf, 0, sizeof(double) * (size_t)npad * S_BLK, s));
+    auto apply = [&](const double*, double* W) -> rfx_status {
         dgemm_bv_kernel<<<dim3(nt, ksn), 128, DB_SMEM, s>>>(B, nt, Vf, n, kchunk, Wpart, c->d_err);
-        bv_reduce_kernel<<<(unsigned)(((size_t)n * S_BLK + 255) / 256), 256, 0, s>>>(Wpart, n, ksn, W);
-        c->launches += 3;
+        if (W) bv_reduce_kernel<<<(unsigned)(((size_t)n * S_BLK + 255) / 256), 256, 0, s>>>(Wpart, n, ksn, W);
+        c->launches += W ? 2 : 1;
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
     };
     // Chebyshev degree 8; up to 4000 products (the eigenvalue-change
     // criterion of 1e-14 ends it far earlier unless the third eigenvalue sits
     // in a tight cluster)
-    return subspace_topk(c, n, 3, apply, 4000, d_coords, evals, 12345, 1e-14, nullptr, nullptr, nullptr, false, 8);
+    return subspace_topk(c, n, 3, apply, 4000, d_coords, evals, 12345, 1e-14, nullptr, nullptr, nullptr, false, 8, Vf,
+                         Wpart, ksn);
 }
 
 }  // namespace rfx
