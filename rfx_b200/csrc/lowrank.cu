@@ -192,8 +192,11 @@ __global__ void pack_x_fp8_kernel(const float* __restrict__ V, const float* __re
 // warps.  A key that lies inside one chunk is written to G directly; a key that
 // crosses a chunk boundary leaves FP32 partial sums (Pf: the chunk's first key,
 // Pl: its last key) that segsum_fix_kernel adds up in chunk order.  Rows move
-// as 16-byte chunks (lane l owns chunks l and l + 32).  G rows of empty keys
-// must be zero beforehand.
+// as 16-byte chunks (lane l owns chunk l, and with TWO also l + 32).  G rows of
+// empty keys are neither written nor read.  Bound by instructions and the
+// latency of a key's turn, not by L2 (28 %): the keys' ends sit in registers
+// (n = 100,000 / 500 trees / W = 96 FP32: 2.83 -> 2.00 ms; W = 160 BF16, n =
+// 50,000 / 1,000 trees: 2.06 -> 1.27 ms).
 constexpr int SEG_CH = 64;
 
 // adds the row (times its scale sc, for FP8 rows) to the lane's sums
@@ -278,7 +281,7 @@ __device__ __forceinline__ void add_partial(const float* in, int lane, bool c0ok
     }
 }
 
-template <typename T, int E>
+template <typename T, int E, bool TWO>
 __global__ void segsum_kernel(const T* __restrict__ X, int n, int W, const int32_t* __restrict__ memb,
                               const int32_t* __restrict__ segoff, const int64_t* __restrict__ segbase, int t0,
                               int t1, int cpt, const int64_t* __restrict__ gofs, T* __restrict__ G,
@@ -298,23 +301,30 @@ __global__ void segsum_kernel(const T* __restrict__ X, int n, int W, const int32
         return;
     }
     const int ce = min(cs + SEG_CH, ntot);
-    // key holding position cs: the largest k with so[k] <= cs (so[0] = 0)
-    int lo = 0, hi = K;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(so + mid) <= cs) lo = mid;
-        else hi = mid;
-    }
-    int key = lo;
-    if (lane == 0) fk[warp] = key;
     const int32_t* mt = memb + (size_t)t * n;
     const int m0 = cs + lane < ce ? __ldg(mt + cs + lane) : 0;
     const int m1 = cs + 32 + lane < ce ? __ldg(mt + cs + 32 + lane) : 0;
+    // key holding position cs: the largest k with so[k] <= cs (so[0] = 0), by a
+    // 32-way search
+    int lo = 0, hi = K;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5;
+        const int c = lo + lane * step;
+        const unsigned le = __ballot_sync(0xffffffffu, c < hi && __ldg(so + c) <= cs);
+        lo += (__popc(le) - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    if (lane == 0) fk[warp] = lo;
+    // the ends of the next 64 keys in registers, so that a key's end does not
+    // wait for memory
+    int kb = lo, key = lo;
+    int e0 = __ldg(so + min(kb + lane + 1, K)), e1 = __ldg(so + min(kb + lane + 33, K));
+    int kend = __shfl_sync(0xffffffffu, e0, 0);
+    bool starts = __ldg(so + lo) >= cs;  // the key starts in this chunk
     const int CH = W / E;
-    const bool c0ok = lane < CH, c1ok = lane + 32 < CH;
+    const bool c0ok = lane < CH, c1ok = TWO && lane + 32 < CH;
     int pos = cs;
     while (pos < ce) {
-        const int kbeg = __ldg(so + key), kend = __ldg(so + key + 1);
         const int e = min(kend, ce);
         float a0[E], a1[E];
 #pragma unroll
@@ -325,7 +335,7 @@ __global__ void segsum_kernel(const T* __restrict__ X, int n, int W, const int32
             const int j = __shfl_sync(0xffffffffu, r < 32 ? m0 : m1, r & 31);
             add_row<T, E>(X + (size_t)j * W, is_fp8<T>() ? __ldg(xs + j) : 1.0f, lane, c0ok, c1ok, a0, a1);
         }
-        if (kbeg >= cs && kend <= ce) {
+        if (starts && kend <= ce) {
             store_grow<T, E>(G + (size_t)(gofs[tb] + key) * W, gs + gofs[tb] + key, lane, c0ok, c1ok, a0, a1);
         } else if (pos == cs) {
             store_partial<T, E>(Pf + (size_t)warp * W, lane, c0ok, c1ok, a0, a1);
@@ -333,10 +343,18 @@ __global__ void segsum_kernel(const T* __restrict__ X, int n, int W, const int32
             store_partial<T, E>(Pl + (size_t)warp * W, lane, c0ok, c1ok, a0, a1);
         }
         pos = e;
-        if (pos < ce) {
-            ++key;
-            while (__ldg(so + key + 1) <= pos) ++key;  // skip empty keys; pos < ntot = so[K] bounds key < K
+        if (pos == ce) break;
+        starts = true;
+        // the next key with members: the first whose end lies past pos
+        int cnt = __popc(__ballot_sync(0xffffffffu, e0 <= pos)) + __popc(__ballot_sync(0xffffffffu, e1 <= pos));
+        while (cnt == 64) {
+            kb += 64;
+            e0 = __ldg(so + min(kb + lane + 1, K));
+            e1 = __ldg(so + min(kb + lane + 33, K));
+            cnt = __popc(__ballot_sync(0xffffffffu, e0 <= pos)) + __popc(__ballot_sync(0xffffffffu, e1 <= pos));
         }
+        key = kb + cnt;
+        kend = __shfl_sync(0xffffffffu, cnt < 32 ? e0 : e1, cnt & 31);
     }
 }
 
@@ -436,7 +454,7 @@ __global__ void segsum_slot_kernel(const T* __restrict__ X, int n, int W, const 
                 amax = fmaxf(amax, __shfl_sync(0xffffffffu, amax, min(31, slot * LPR + (lr + d) % LPR)));
             scale = amax > 0.0f ? 448.0f / amax : 1.0f;
         }
-        if (cntm == 0) continue;  // empty key: its zero row was cleared beforehand
+        if (cntm == 0) continue;  // empty key
         if (whole) {
             T* gr = G + (size_t)(gofs[tb] + k) * W;
 #pragma unroll
@@ -493,32 +511,43 @@ __global__ void segsum_fix_kernel(int n, int W, const int32_t* __restrict__ sego
 }
 
 // Y[i] (+)= sum over trees [t0, t1) of G_t[key_t(i) ^ 1]; one warp per sample,
-// 16-byte chunks per lane, 32 trees' keys fetched at once.
-template <typename T, int E>
-__global__ void pull_kernel(const T* __restrict__ G, const int32_t* __restrict__ key, int n, int W, int t0, int t1,
-                            const int64_t* __restrict__ gofs, float* __restrict__ Y, int accumulate,
+// 16-byte chunks per lane, 32 trees' keys fetched at once.  Leaving out the keys
+// without members saves their rows here and clearing G beforehand (n = 50,000
+// / 1,000 trees / W = 160 BF16: 1.57 + 0.56 ms before, 1.07 now); the next 32
+// trees' rows are found while the current ones' are added (n = 100,000 / 500
+// trees / W = 96 FP32: 2.18 -> 1.64 ms).
+template <typename T, int E, bool TWO>
+__global__ void pull_kernel(const T* __restrict__ G, const int32_t* __restrict__ key,
+                            const int32_t* __restrict__ segoff, const int64_t* __restrict__ segbase, int n, int W,
+                            int t0, int t1, const int64_t* __restrict__ gofs, float* __restrict__ Y, int accumulate,
                             const float* __restrict__ gs) {
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= n) return;
     const int i = (int)warp;
     const int CH = W / E;
-    const bool c0ok = lane < CH, c1ok = lane + 32 < CH;
+    const bool c0ok = lane < CH, c1ok = TWO && lane + 32 < CH;
     float a0[E], a1[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) a0[e] = a1[e] = 0.0f;
+    // the G row that tree t adds, or -1: a key without members has none
+    auto row_of = [&](int t) -> long long {
+        const int k = t < t1 ? __ldg(key + (size_t)t * n + i) : -1;
+        if (k < 0) return -1;
+        const int32_t* so = segoff + segbase[t] + (k ^ 1);
+        return __ldg(so) < __ldg(so + 1) ? gofs[t - t0] + (k ^ 1) : -1;
+    };
+    long long gnext = row_of(t0 + lane);
     for (int tb = t0; tb < t1; tb += 32) {
-        const int t = tb + lane;
-        long long gi = -1;
-        if (t < t1) {
-            const int k = __ldg(key + (size_t)t * n + i);
-            if (k >= 0) gi = gofs[t - t0] + (k ^ 1);
-        }
-        const int cnt = min(32, t1 - tb);
+        const long long gi = gnext;
+        gnext = row_of(tb + 32 + lane);  // with the rows below in flight
+        // the trees that add something, in order
+        unsigned todo = __ballot_sync(0xffffffffu, gi >= 0);
+        const int cnt = __popc(todo);
 #pragma unroll 4
         for (int q = 0; q < cnt; ++q) {
-            const long long r = __shfl_sync(0xffffffffu, gi, q);
-            if (r < 0) continue;
+            const long long r = __shfl_sync(0xffffffffu, gi, __ffs(todo) - 1);
+            todo &= todo - 1;
             const T* gr = G + (size_t)r * W;
             float v[E];
             if constexpr (is_fp8<T>()) {
@@ -838,16 +867,12 @@ rfx_status apply_m(Ctx* c, const float* V, int w, float* MV, const float* dinv, 
         const int t0 = (int)batch_start[b], t1 = (int)batch_start[b + 1];
         // key prefix of this batch (device copy prepared by the caller)
         const int64_t* gofs = d_gofs + (h_gofs_all[b]);
-        const int64_t keys = h_gofs_all[b + 1] - h_gofs_all[b] - 1;  // stored with one sentinel per batch
-        (void)keys;
-        const int64_t total_keys = c->h_segbase[t1] - c->h_segbase[t0] - (t1 - t0);
         static_assert(std::is_same<TX, TG>::value, "X and the leaf sums share one storage type");
         const int cpt = (n + SEG_CH - 1) / SEG_CH;
         const int64_t chunks = (int64_t)(t1 - t0) * cpt;
-        RFX_CUDA(cudaMemsetAsync(G, 0, sizeof(TG) * (size_t)total_keys * W, s));
-        if constexpr (is_fp8<TG>()) RFX_CUDA(cudaMemsetAsync(gs, 0, sizeof(float) * (size_t)total_keys, s));
-        auto run = [&](auto e_tag) -> rfx_status {
+        auto run = [&](auto e_tag, auto two_tag) -> rfx_status {
             constexpr int E = decltype(e_tag)::value;
+            constexpr bool TWO = decltype(two_tag)::value;
             // shape 0: the warp takes the chunk's keys in turn; 1: slots of
             // the warp take several keys at once
             const int tk = is_fp8<TX>() ? TK_SEGSUM_FP8 : std::is_same<TX, float>::value ? TK_SEGSUM_F32 : TK_SEGSUM_BF16;
@@ -856,7 +881,7 @@ rfx_status apply_m(Ctx* c, const float* V, int w, float* MV, const float* dinv, 
                     segsum_slot_kernel<TX, E, 4><<<nblk(chunks * 32), 256, 0, s>>>(
                         X, n, W, c->d_memb, c->d_segoff, c->d_segbase, t0, t1, cpt, gofs, G, Pf, Pl, fk, xs, gs);
                 else
-                    segsum_kernel<TX, E><<<nblk(chunks * 32), 256, 0, s>>>(X, n, W, c->d_memb, c->d_segoff,
+                    segsum_kernel<TX, E, TWO><<<nblk(chunks * 32), 256, 0, s>>>(X, n, W, c->d_memb, c->d_segoff,
                                                                            c->d_segbase, t0, t1, cpt, gofs, G, Pf,
                                                                            Pl, fk, xs, gs);
                 RFX_CUDA(cudaGetLastError());
@@ -865,18 +890,22 @@ rfx_status apply_m(Ctx* c, const float* V, int w, float* MV, const float* dinv, 
             if (st0 != RFX_OK) return st0;
             segsum_fix_kernel<TG, E><<<nblk(chunks * 32), 256, 0, s>>>(n, W, c->d_segoff, c->d_segbase, t0, t1, cpt,
                                                                        gofs, G, Pf, Pl, fk, gs);
-            pull_kernel<TG, E><<<nblk((int64_t)n * 32), 256, 0, s>>>(G, c->d_key, n, W, t0, t1, gofs, Y, b > 0, gs);
+            pull_kernel<TG, E, TWO><<<nblk((int64_t)n * 32), 256, 0, s>>>(G, c->d_key, c->d_segoff, c->d_segbase, n, W,
+                                                                        t0, t1, gofs, Y, b > 0, gs);
             return RFX_OK;
         };
-        // BF16 rows narrower than 32 16-byte chunks use 8-byte chunks, so more lanes carry data
+        // FP32 rows of more than 128 columns give a lane two chunks; BF16 rows
+        // narrower than 16 16-byte chunks use 8-byte chunks, so more lanes carry data
         rfx_status rs;
+        constexpr std::true_type two{};
+        constexpr std::false_type one{};
         if constexpr (std::is_same<TX, float>::value) {
-            rs = run(std::integral_constant<int, 4>{});
+            rs = W > 128 ? run(std::integral_constant<int, 4>{}, two) : run(std::integral_constant<int, 4>{}, one);
         } else if constexpr (is_fp8<TX>()) {
-            rs = run(std::integral_constant<int, 8>{});
+            rs = run(std::integral_constant<int, 8>{}, one);
         } else {
-            if (W / 8 > 16) rs = run(std::integral_constant<int, 8>{});
-            else rs = run(std::integral_constant<int, 4>{});
+            if (W / 8 > 16) rs = run(std::integral_constant<int, 8>{}, one);
+            else rs = run(std::integral_constant<int, 4>{}, one);
         }
         if (rs != RFX_OK) return rs;
         c->launches += 3;
@@ -982,8 +1011,11 @@ rfx_status lowrank_compute(Ctx* c, int k, int oversample, int power_iters, int p
     RFX_CUDA(cudaMemcpyAsync(d_gofs, h_gofs.data(), sizeof(int64_t) * h_gofs.size(), cudaMemcpyHostToDevice, s));
     RFX_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
     dinv_kernel<<<nblk(n), 256, 0, s>>>(c->d_nout, n, dinv);
-    gauss_kernel<float><<<nblk((int64_t)n * w), 256, 0, s>>>(Om, (int64_t)n * w, seed);
-    c->launches += 2;
+    c->launches += 1;
+    if (!d_apply_in) {
+        gauss_kernel<float><<<nblk((int64_t)n * w), 256, 0, s>>>(Om, (int64_t)n * w, seed);
+        c->launches += 1;
+    }
     // per-batch prefix pointers: apply_m takes the whole table and indexes it
     std::vector<int64_t> pref_at(gofs_index.begin(), gofs_index.end());
     auto apply = [&](const float* V, float* MV, bool fp32) -> rfx_status {
