@@ -120,9 +120,7 @@ void free_forest(Ctx* c) {
     dfree(c, c->d_sqsd); dfree(c, c->d_opp); dfree(c, c->d_order);
     dfree(c, c->d_hubflag); dfree(c, c->d_hubtiles); dfree(c, c->d_hubstate);
     dfree(c, c->d_nin); dfree(c, c->d_tnodewt);
-    dfree(c, c->d_lrA); dfree(c, c->d_lrAq); dfree(c, c->d_lrScale);
-    if (c->d_lrQ) cudaFree(c->d_lrQ);
-    c->d_lrQ = nullptr;
+    dfree(c, c->d_lrA); dfree(c, c->d_lrAq); dfree(c, c->d_lrScale); dfree(c, c->d_lrQ);
     c->lr_rank = 0;
     c->lr_qformat = 0;
     c->loaded = c->routed = c->csr_built = false;
@@ -1153,8 +1151,7 @@ rfx_status rfx_lowrank(rfx_ctx* ctx, const rfx_lowrank_opts* o, float* A, float*
     dfree(c, c->d_lrA);
     dfree(c, c->d_lrAq);
     dfree(c, c->d_lrScale);
-    if (c->d_lrQ) cudaFree(c->d_lrQ);
-    c->d_lrQ = nullptr;
+    dfree(c, c->d_lrQ);
     c->lr_rank = 0;
     c->lr_qformat = 0;
     if ((st = dalloc(c, &c->d_lrA, (size_t)c->n * k))) return st;
@@ -1232,13 +1229,8 @@ rfx_status rfx_lowrank_quantize(rfx_ctx* ctx, int format, void* q, float* scales
     const size_t nk = (size_t)c->n * k;
     // stored bytes: INT8 / FP8 one per entry, NF4 half, FP16 two
     const size_t qbytes = format == 3 ? (nk + 1) / 2 : format == 4 ? 2 * nk : nk;
-    if (c->d_lrQ) cudaFree(c->d_lrQ);
-    c->d_lrQ = nullptr;
-    if (ctx_malloc(c, (void**)&c->d_lrQ, qbytes) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("rfx_lowrank_quantize: allocation failed");
-        return RFX_ERR_OOM;
-    }
+    dfree(c, c->d_lrQ);
+    if ((st = dalloc(c, &c->d_lrQ, qbytes))) return st;
     if ((st = dalloc(c, &c->d_lrScale, k))) return st;
     if ((st = dalloc(c, &c->d_lrAq, nk))) return st;
     if ((st = lowrank_quantize(c, c->d_lrA, k, format, c->d_lrQ, c->d_lrScale))) return st;
@@ -1326,16 +1318,18 @@ rfx_status rfx_outlier_scores(rfx_ctx* ctx, int use_quantized, float* scores) {
         set_error("rfx_outlier_scores: factors not available");
         return RFX_ERR_STATE;
     }
-    float* d = nullptr;
-    cudaError_t e = ctx_malloc(c, (void**)&d, sizeof(float) * c->n);
-    if (e != cudaSuccess) return cuda_fail(e, "rfx_outlier_scores");
+    Scratch sc(c);
+    float* d = sc.get<float>((size_t)c->n);
+    if (!d) {
+        set_error("rfx_outlier_scores: device allocation failed");
+        return RFX_ERR_OOM;
+    }
     st = launch_outlier_scores(c, dA, c->lr_rank, d);
     std::vector<float> h(c->n);
     if (st == RFX_OK) {
-        e = cudaMemcpy(h.data(), d, sizeof(float) * c->n, cudaMemcpyDeviceToHost);
+        const cudaError_t e = cudaMemcpy(h.data(), d, sizeof(float) * c->n, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) st = cuda_fail(e, "rfx_outlier_scores D2H");
     }
-    cudaFree(d);
     if (st) return st;
     // normalise by the median element sorted[n/2], as compute_outlier_scores does
     std::vector<float> srt = h;

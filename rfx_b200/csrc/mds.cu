@@ -959,20 +959,63 @@ __global__ void subtract_mean_kernel(double* __restrict__ W, const double* __res
 // diagonal: sum_j P_ij^2 = 1 + (a_i^T (A^T A) a_i - |a_i|^4)  (exact algebra of
 // the factor form; compute_outlier_scores, src/rf_random_forest.cpp:2489-2520,
 // on the full matrix).
-__global__ void outlier_raw_kernel(const float* __restrict__ A, const double* __restrict__ AtA, int n, int k,
-                                   float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// 32 rows per CTA; thread (row, g) forms (A^T A a_i)_a for eight a at a time,
+// operands from shared memory (a warp's lanes are rows, so A^T A is read by
+// broadcast), then one thread per row adds the k products in order.
+// n = 50,000 / k = 64: 79 us (1,165 us with one thread per row reading both
+// operands through L1 and converting A for every product).
+constexpr int OR_ROWS = 32;
+__host__ __device__ inline size_t outlier_smem(int k) {
+    const int kp = (k + 7) & ~7;
+    return sizeof(double) * ((size_t)k * kp + 2 * (size_t)k * OR_ROWS);
+}
+__global__ void __launch_bounds__(256) outlier_raw_kernel(const float* __restrict__ A, const double* __restrict__ AtA,
+                                                          int n, int k, float* __restrict__ out) {
+    extern __shared__ __align__(16) double or_sm[];
+    const int kp = (k + 7) & ~7;
+    double* M = or_sm;                    // M[b][a] = AtA[a][b], a padded to kp with zeros
+    double* X = M + (size_t)k * kp;       // X[b][row]
+    double* V = X + (size_t)k * OR_ROWS;  // V[a][row]
+    const int i0 = blockIdx.x * OR_ROWS, rows = min(OR_ROWS, n - i0);
+    for (int e = threadIdx.x; e < k * kp; e += 256) {
+        const int b = e / kp, a = e % kp;
+        M[e] = a < k ? AtA[(size_t)a * k + b] : 0.0;
+    }
+    for (int e = threadIdx.x; e < rows * k; e += 256) {
+        const int r = e / k, b = e % k;
+        X[b * OR_ROWS + r] = (double)A[(size_t)i0 * k + e];
+    }
+    __syncthreads();
+    const int row = threadIdx.x & 31, g = threadIdx.x >> 5;
+    for (int a0 = g * 8; a0 < k; a0 += 64) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = 0.0;
+#pragma unroll 4
+        for (int b = 0; b < k; ++b) {
+            const double x = X[b * OR_ROWS + row];
+            const double2* m = reinterpret_cast<const double2*>(M + (size_t)b * kp + a0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double2 mm = m[u];
+                v[2 * u] = fma(mm.x, x, v[2 * u]);
+                v[2 * u + 1] = fma(mm.y, x, v[2 * u + 1]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (a0 + u < k) V[(a0 + u) * OR_ROWS + row] = v[u];
+    }
+    __syncthreads();
+    if (g != 0 || row >= rows) return;
     double q = 0.0, nrm = 0.0;
     for (int a = 0; a < k; ++a) {
-        const double x = A[(size_t)i * k + a];
-        nrm += x * x;
-        double v = 0.0;
-        for (int b = 0; b < k; ++b) v += AtA[a * k + b] * (double)A[(size_t)i * k + b];
-        q += x * v;
+        const double x = X[a * OR_ROWS + row];
+        nrm = fma(x, x, nrm);
+        q = fma(x, V[a * OR_ROWS + row], q);
     }
     const double ss = 1.0 + (q - nrm * nrm);
-    out[i] = (float)(1.0 / ss);
+    out[i0 + row] = (float)(1.0 / ss);
 }
 
 // Partial A^T A over the rows blockIdx.x, blockIdx.x + gridDim.x, ... into
@@ -1139,7 +1182,9 @@ rfx_status launch_outlier_scores(Ctx* c, const float* dA, int k, float* d_out) {
     if (!AtA || !apart) return RFX_ERR_OOM;
     ata_kernel<<<dim3(256, (k * k + 255) / 256), 256, 0, s>>>(dA, n, k, apart);
     part_sum_kernel<double><<<(k * k * 32 + 255) / 256, 256, 0, s>>>(apart, 256, k * k, 1.0, AtA);
-    outlier_raw_kernel<<<(n + 255) / 256, 256, 0, s>>>(dA, AtA, n, k, d_out);
+    RFX_CUDA(cudaFuncSetAttribute(outlier_raw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)outlier_smem(k)));
+    outlier_raw_kernel<<<(n + OR_ROWS - 1) / OR_ROWS, 256, outlier_smem(k), s>>>(dA, AtA, n, k, d_out);
     c->launches += 3;
     RFX_CUDA(cudaGetLastError());
     RFX_CUDA(cudaStreamSynchronize(s));

@@ -120,7 +120,7 @@ struct Ctx {
     // low-rank factors (P ~= I + A A^T)
     float* d_lrA = nullptr;             // n*lr_rank FP32
     float* d_lrAq = nullptr;            // n*lr_rank dequantised copy
-    void* d_lrQ = nullptr;              // n*lr_rank quantised (int8 or fp8)
+    uint8_t* d_lrQ = nullptr;           // the stored codes (INT8, FP8, NF4 or FP16)
     float* d_lrScale = nullptr;         // lr_rank per-column scales
     int lr_rank = 0;
     int lr_qformat = 0;                 // 0 none, 1 INT8, 2 FP8 e4m3
