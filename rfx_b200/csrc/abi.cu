@@ -493,6 +493,9 @@ static rfx_status load_forest(Ctx* c, const LoadInput& in) {
             c->max_keys = std::max(c->max_keys, 2 * nleaf[t]);
             c->max_nnode = std::max(c->max_nnode, nnode[t]);
         }
+        int most_levels = 0;
+        for (int m = 0; m < p; ++m) most_levels = std::max(most_levels, in.cat[m]);
+        c->plain_walks = !in.has_catgoleft && most_levels <= (1 << 20) && c->max_nnode <= 2 * n + 1;
         ALLOC(d_segoff, segbase[T]);
 #undef ALLOC
         if (st != RFX_OK) {

@@ -61,7 +61,9 @@ pack_nodes_kernel(const int64_t* __restrict__ offs, const int32_t* __restrict__ 
                 if (l < 0 || l >= nn || r < 0 || r >= nn) load_fail(err, 3, t, k);
             }
             DNode d;
-            d.split = split[g];
+            // (a categorical split has no threshold: its record holds the end of
+            // the values that round to a level, level count + 1/2)
+            d.split = catf ? (float)cat[bv] + 0.5f : split[g];
             d.left = l;
             d.right = r;
             d.meta = (var & 0xffff) | ((st & 0xff) << 16) | (catf << 24);

@@ -14,7 +14,8 @@
 namespace rfx {
 
 // Device node record (16 bytes, one int4 load per traversal step):
-//   x = split threshold (float bits), y = left child, z = right child,
+//   x = split threshold (float bits; of a categorical split level count + 1/2),
+//   y = left child, z = right child,
 //   w = var (bits 0..15) | status as int8 (bits 16..23) | categorical (bit 24).
 // Node ids are local to their tree.
 struct __align__(16) DNode {
@@ -65,6 +66,7 @@ struct Ctx {
     int max_keys = 0;                   // max_t 2*nleaf_t
     int max_nnode = 0;
     int iv_words = 0;                   // ceil(p / 64)
+    bool plain_walks = false;           // see walk_terminal_plain (walks.cuh)
 
     float* d_X = nullptr;               // n*p
     int32_t* d_y = nullptr;             // n

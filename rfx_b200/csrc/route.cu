@@ -7,6 +7,8 @@
 //                                          cpu_proximity, src/rf_proximity.cpp:114-136).
 // Grid: x = sample chunk, y = tree, so CTAs resident at the same time work on
 // the same few trees and their node arrays stay in L2.
+#include <algorithm>
+
 #include "walks.cuh"
 
 namespace rfx {
@@ -16,7 +18,7 @@ namespace {
 // Launch shapes the autotuner chooses from: threads per CTA x trees per
 // thread (a thread walks TPC consecutive trees for its sample, reusing the
 // sample's feature row from L1).
-template <int RT, int TPC>
+template <int RT, int TPC, bool PLAIN>
 __global__ void __launch_bounds__(RT)
 route_kernel(const float* __restrict__ X, int n, int p, int T, int nclass, const DNode* __restrict__ nodes,
              const int32_t* __restrict__ nodeclass, const int32_t* __restrict__ leafidx,
@@ -41,10 +43,12 @@ route_kernel(const float* __restrict__ X, int n, int p, int T, int nclass, const
         int node;
         if (!ib) {
             int cls;
-            node = walk_testreebag(xrow, p, tn, tc, nn, cat, cgl, maxcat, &cls);
+            node = PLAIN ? walk_testreebag_plain(GlobalRow{xrow}, tn, tc, &cls)
+                         : walk_testreebag(xrow, p, tn, tc, nn, cat, cgl, maxcat, &cls);
             if (cls >= 0 && cls < nclass) atomicAdd(votes + (size_t)i * nclass + cls, 1);
         } else {
-            node = walk_terminal(xrow, p, tn, cat, cgl, maxcat, 2 * n + 1);
+            node = PLAIN ? walk_terminal_plain(GlobalRow{xrow}, tn, 2 * n + 1)
+                         : walk_terminal(xrow, p, tn, cat, cgl, maxcat, 2 * n + 1);
         }
         const int li = (node >= 0 && node < nn) ? __ldg(leafidx + o + node) : -1;
         key_out[ti] = li >= 0 ? 2 * li + (ib ? 1 : 0) : -1;
@@ -216,7 +220,7 @@ route2_kernel(const float* __restrict__ X, int n, int p, int T, int nclass, cons
 // result is indexed by sample, so only the order of work changes.  With PF
 // the walks load both children of each split node with the feature value
 // (walk_testreebag_pf / walk_terminal_pf).
-template <int RT, bool PF = false>
+template <int RT, bool PF = false, bool PLAIN = false>
 __global__ void __launch_bounds__(RT)
 route_leaf_order_kernel(const float* __restrict__ X, int n, int p, int nclass, const DNode* __restrict__ nodes,
                         const int32_t* __restrict__ nodeclass, const int32_t* __restrict__ leafidx,
@@ -240,11 +244,13 @@ route_leaf_order_kernel(const float* __restrict__ X, int n, int p, int nclass, c
     int node;
     if (!ib) {
         int cls;
-        if constexpr (PF) node = walk_testreebag_pf(GlobalRow{xrow}, p, tn, tc, nn, cat, cgl, maxcat, &cls);
+        if constexpr (PLAIN) node = walk_testreebag_plain(GlobalRow{xrow}, tn, tc, &cls);
+        else if constexpr (PF) node = walk_testreebag_pf(GlobalRow{xrow}, p, tn, tc, nn, cat, cgl, maxcat, &cls);
         else node = walk_testreebag(xrow, p, tn, tc, nn, cat, cgl, maxcat, &cls);
         if (cls >= 0 && cls < nclass) atomicAdd(votes + (size_t)i * nclass + cls, 1);
     } else {
-        if constexpr (PF) node = walk_terminal_pf(GlobalRow{xrow}, p, tn, cat, cgl, maxcat, 2 * n + 1);
+        if constexpr (PLAIN) node = walk_terminal_plain(GlobalRow{xrow}, tn, 2 * n + 1);
+        else if constexpr (PF) node = walk_terminal_pf(GlobalRow{xrow}, p, tn, cat, cgl, maxcat, 2 * n + 1);
         else node = walk_terminal(xrow, p, tn, cat, cgl, maxcat, 2 * n + 1);
     }
     const int li = (node >= 0 && node < nn) ? __ldg(leafidx + o + node) : -1;
@@ -348,6 +354,7 @@ constexpr int ROUTE_SHAPES = 10;
 
 // votes must be zero beforehand (the kernel adds to them)
 void route_launch(Ctx* c, int shape, int32_t* d_leaf) {
+    const bool plain = c->plain_walks;  // shapes 0-4
     auto go = [&](auto kernel, int rt, int tpc) {
         dim3 grid((c->n + rt - 1) / rt, (c->T + tpc - 1) / tpc);
         kernel<<<grid, rt, 0, c->stream>>>(c->d_X, c->n, c->p, c->T, c->nclass, c->d_nodes, c->d_nodeclass,
@@ -361,16 +368,16 @@ void route_launch(Ctx* c, int shape, int32_t* d_leaf) {
                                            c->d_catgoleft, c->maxcat, c->d_key, d_leaf, c->d_votes);
     };
     switch (shape) {
-        case 1: go(route_kernel<128, 1>, 128, 1); break;
-        case 2: go(route_kernel<512, 1>, 512, 1); break;
-        case 3: go(route_kernel<256, 2>, 256, 2); break;
-        case 4: go(route_kernel<256, 4>, 256, 4); break;
+        case 1: plain ? go(route_kernel<128, 1, true>, 128, 1) : go(route_kernel<128, 1, false>, 128, 1); break;
+        case 2: plain ? go(route_kernel<512, 1, true>, 512, 1) : go(route_kernel<512, 1, false>, 512, 1); break;
+        case 3: plain ? go(route_kernel<256, 2, true>, 256, 2) : go(route_kernel<256, 2, false>, 256, 2); break;
+        case 4: plain ? go(route_kernel<256, 4, true>, 256, 4) : go(route_kernel<256, 4, false>, 256, 4); break;
         case 5: go(route2_kernel<256, 2>, 256, 2); break;
         case 6: go(route2_kernel<256, 4>, 256, 4); break;
         case 7: go(route2_kernel<128, 4>, 128, 4); break;
         case 8: go_nodes(route_nodes_kernel<256, 8, 2048>, 256, 8); break;
         case 9: go_nodes(route_nodes_kernel<256, 4, 1024>, 256, 4); break;
-        default: go(route_kernel<256, 1>, 256, 1); break;
+        default: plain ? go(route_kernel<256, 1, true>, 256, 1) : go(route_kernel<256, 1, false>, 256, 1); break;
     }
 }
 
@@ -440,20 +447,81 @@ __global__ void oob_error_kernel(const unsigned int* __restrict__ counts, float*
     *err = total > 0 ? __fsub_rn(1.0f, __fdiv_rn((float)correct, (float)total)) : 0.0f;
 }
 
-constexpr int PRED_THREADS = 256;
+// Test-set votes.  A CTA takes 32 SW samples and a run of trees, TW of them at
+// a time (warp w: samples 32 (w % SW) + lane, trees w / SW, w / SW + TW, ...),
+// counts in shared memory and adds each count to the votes once (or stores it,
+// where one run holds all trees).  With one warp per tree and 32 samples the
+// smallest calls spread over the GPU; large ones take 512 samples, whose
+// features then stay in L1 over the run.  Walks are short here (a categorical
+// split ends most), so the bound was the L1 tag stage (one line per lane and
+// feature, 87 % busy): XT reads a transposed copy, one line for the lanes at a
+// node (a third of the accesses), PLAIN drops the tests the load has made.
+// m = 50,000 / 1,000 trees / p = 54: 0.98 -> 0.86 ms; now bound by divergence
+// (13 of 32 lanes active), not memory.
+template <int SW, int TW, bool XT, bool PLAIN>
+__global__ void __launch_bounds__(SW * TW * 32)
+predict_kernel(const float* __restrict__ X, int m, int ms, int p, int nclass, int maxnode, int T, int run,
+               const DNode* __restrict__ nodes, const int32_t* __restrict__ nodeclass,
+               const int64_t* __restrict__ offs, const int32_t* __restrict__ cat,
+               const int32_t* __restrict__ catgoleft, int maxcat, int32_t* __restrict__ votes) {
+    extern __shared__ int32_t s_votes[];  // 32 SW x nclass
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sl = (w % SW) * 32 + lane;
+    const int s0 = blockIdx.x * 32 * SW, s = s0 + sl;
+    const int cells = min(32 * SW, m - s0) * nclass;
+    for (int e = threadIdx.x; e < cells; e += SW * TW * 32) s_votes[e] = 0;
+    __syncthreads();
+    if (s < m) {
+        const GlobalRow xg{X + (size_t)s * p};
+        const ColumnRow xc{X + s, (size_t)ms};
+        const int t1 = min(T, (int)(blockIdx.y + 1) * run);
+        for (int t = blockIdx.y * run + w / SW; t < t1; t += TW) {
+            const int64_t o = offs[t];
+            const int32_t* cgl = catgoleft ? catgoleft + o * maxcat : nullptr;
+            const int c = PLAIN ? (XT ? walk_predict_plain(xc, nclass, nodes + o, nodeclass + o, maxnode)
+                                      : walk_predict_plain(xg, nclass, nodes + o, nodeclass + o, maxnode))
+                          : XT ? walk_predict(xc, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode)
+                             : walk_predict(xg, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode);
+            if (c < 0) continue;
+            if (TW == 1) s_votes[sl * nclass + c] += 1;
+            else atomicAdd(s_votes + sl * nclass + c, 1);
+        }
+    }
+    __syncthreads();
+    int32_t* out = votes + (size_t)s0 * nclass;
+    for (int e = threadIdx.x; e < cells; e += SW * TW * 32) {
+        if (gridDim.y == 1) out[e] = s_votes[e];
+        else if (s_votes[e]) atomicAdd(out + e, s_votes[e]);
+    }
+}
 
+// The same with an atomic per walk, for more classes than shared memory holds.
+constexpr int PRED_THREADS = 256;
 __global__ void __launch_bounds__(PRED_THREADS)
-predict_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode, const DNode* __restrict__ nodes,
-               const int32_t* __restrict__ nodeclass, const int64_t* __restrict__ offs,
-               const int32_t* __restrict__ cat, const int32_t* __restrict__ catgoleft, int maxcat,
-               int32_t* __restrict__ votes) {
+predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode,
+                      const DNode* __restrict__ nodes, const int32_t* __restrict__ nodeclass,
+                      const int64_t* __restrict__ offs, const int32_t* __restrict__ cat,
+                      const int32_t* __restrict__ catgoleft, int maxcat, int32_t* __restrict__ votes) {
     const int t = blockIdx.y;
     const int s = blockIdx.x * PRED_THREADS + threadIdx.x;
     if (s >= m) return;
     const int64_t o = offs[t];
-    const int c = walk_predict(X + (size_t)s * p, p, nclass, nodes + o, nodeclass + o, cat,
+    const int c = walk_predict(GlobalRow{X + (size_t)s * p}, p, nclass, nodes + o, nodeclass + o, cat,
                                catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
     if (c >= 0) atomicAdd(votes + (size_t)s * nclass + c, 1);
+}
+
+// XT = X transposed (p x m, row stride ms).
+__global__ void __launch_bounds__(256)
+transpose_kernel(const float* __restrict__ X, int m, int p, int ms, float* __restrict__ XT) {
+    __shared__ float tile[32][33];
+    const int i0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8)
+        if (i0 + r < m && c0 + tx < p) tile[r][tx] = X[(size_t)(i0 + r) * p + c0 + tx];
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8)
+        if (c0 + r < p && i0 + tx < m) XT[(size_t)(c0 + r) * ms + i0 + tx] = tile[tx][r];
 }
 
 }  // namespace
@@ -500,6 +568,10 @@ rfx_status launch_route(Ctx* c) {
                 if (srt == 64) go(route_leaf_staged_kernel<64>, 64, sm);
                 else if (srt == 128) go(route_leaf_staged_kernel<128>, 128, sm);
                 else go(route_leaf_staged_kernel<256>, 256, sm);
+            } else if (c->plain_walks) {
+                if (shape == 0 || shape == 4) go(route_leaf_order_kernel<128, false, true>, 128, 0);
+                else if (shape == 2) go(route_leaf_order_kernel<512, false, true>, 512, 0);
+                else go(route_leaf_order_kernel<256, false, true>, 256, 0);
             } else if (shape == 0 || shape == 4) {
                 go(route_leaf_order_kernel<128>, 128, 0);
             } else if (shape == 2) {
@@ -562,12 +634,53 @@ rfx_status launch_oob_summary_f32(Ctx* c, const float* d_q, float* d_errout, int
 
 rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
     StageTimer st(c, ST_PREDICT, m > 0 ? 1 : 0);
-    RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * c->nclass, c->stream));
     if (m == 0) return RFX_OK;
-    dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, c->T);
-    predict_kernel<<<grid, PRED_THREADS, 0, c->stream>>>(dX, m, c->p, c->nclass, 2 * c->n + 1, c->d_nodes,
-                                                         c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft,
-                                                         c->maxcat, d_votes);
+    const int T = c->T, nc = c->nclass;
+    const size_t row = 32 * (size_t)nc * sizeof(int32_t);
+    const int ms = (m + 31) & ~31;
+    // from 4,096 rows on (and where 512 samples' counts fit) the features are
+    // read from a transposed copy (made here, 5 us at 50,000 x 54; without room
+    // for it from the rows): the lanes of a warp hold consecutive samples, so
+    // one line serves all lanes at a node
+    Scratch sc(c);
+    const bool large = m >= 4096 && 16 * row <= 96 * 1024;
+    float* XT = large ? sc.get<float>((size_t)ms * c->p) : nullptr;
+    if (XT) {
+        transpose_kernel<<<dim3((m + 31) / 32, (c->p + 31) / 32), 256, 0, c->stream>>>(dX, m, c->p, ms, XT);
+        RFX_CUDA(cudaGetLastError());
+        c->launches += 1;
+    }
+    auto go = [&](auto kernel, int sw, int tw) -> rfx_status {
+        // runs of trees: enough CTAs for about eight rounds over the SMs, each
+        // warp at least one tree
+        const int cols = (m + 32 * sw - 1) / (32 * sw);
+        const int want = std::max(1, (int)(8ll * 148 * 8 / (sw * tw) / cols));
+        const int per = (T + tw - 1) / tw;  // a warp's trees if one CTA took all
+        const int run = tw * ((per + std::min(want, per) - 1) / std::min(want, per));
+        const int runs = (T + run - 1) / run;
+        if (runs > 1) RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
+        const size_t smem = row * sw;
+        if (smem > 48 * 1024)
+            RFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<dim3(cols, runs), sw * tw * 32, smem, c->stream>>>(
+            XT ? XT : dX, m, ms, c->p, nc, 2 * c->n + 1, T, run, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat,
+            c->d_catgoleft, c->maxcat, d_votes);
+        RFX_CUDA(cudaGetLastError());
+        return RFX_OK;
+    };
+    const bool plain = c->plain_walks;
+    if (large) {
+        if (XT)
+            return plain ? go(predict_kernel<16, 2, true, true>, 16, 2) : go(predict_kernel<16, 2, true, false>, 16, 2);
+        return plain ? go(predict_kernel<16, 2, false, true>, 16, 2) : go(predict_kernel<16, 2, false, false>, 16, 2);
+    }
+    if (row <= 96 * 1024)
+        return plain ? go(predict_kernel<1, 8, false, true>, 1, 8) : go(predict_kernel<1, 8, false, false>, 1, 8);
+    RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
+    dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, T);
+    predict_direct_kernel<<<grid, PRED_THREADS, 0, c->stream>>>(dX, m, c->p, nc, 2 * c->n + 1, c->d_nodes,
+                                                                c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft,
+                                                                c->maxcat, d_votes);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }

@@ -52,6 +52,12 @@ struct GlobalRow {
     const float* r;
     __device__ __forceinline__ float operator()(int m) const { return __ldg(r + m); }
 };
+// One sample's column of a feature-major table (row stride ms).
+struct ColumnRow {
+    const float* c;
+    size_t ms;
+    __device__ __forceinline__ float operator()(int m) const { return __ldg(c + m * ms); }
+};
 struct SharedRow {
     const float* r;
     __device__ __forceinline__ float operator()(int m) const { return r[m]; }
@@ -258,12 +264,81 @@ __device__ __forceinline__ int walk_terminal(const float* __restrict__ xrow, int
     return walk_terminal_src(xrow, p, GlobalNodes{nodes}, cat, cgl, maxcat, maxnode);
 }
 
+// The walks without a go-left table (the reference's CPU grower leaves it
+// zero): every categorical split then sends right.  testreebag takes any value
+// there; the other two rules stop at the root (class 0) unless v rounds to a
+// level, 0.5 <= v < level count + 1/2, which the record's split holds.  What the
+// forest load has checked (features and children of non-terminal nodes in
+// range) is not tested again; plain_walks also asks for level counts that are
+// exact in FP32 and for no tree beyond the rules' bound of 2n + 1 nodes.  About
+// half the instructions of the general walks.
+template <typename XR>
+__device__ __forceinline__ int walk_testreebag_plain(const XR& xrow, const DNode* __restrict__ nodes,
+                                                     const int32_t* __restrict__ nclass_of, int* cls) {
+    int kt = 0;
+    DNode nd = load_node(nodes, 0);
+    for (int steps = 1; node_status(nd.meta) == 1 && steps < 1000; ++steps) {
+        const bool left = !node_cat(nd.meta) && xrow(node_var(nd.meta)) <= nd.split;
+        kt = left ? nd.left : nd.right;
+        nd = load_node(nodes, kt);
+    }
+    const int st = node_status(nd.meta);
+    if (st != -1 && st != 2) kt = 0;
+    *cls = __ldg(nclass_of + kt);
+    return kt;
+}
+
+// One step of the other two rules: the child, or -1 where they stop.
+__device__ __forceinline__ int step_plain(const DNode& nd, float v) {
+    const bool cat = node_cat(nd.meta);
+    if (cat && !(v >= 0.5f && v < nd.split)) return -1;
+    return !cat && v <= nd.split ? nd.left : nd.right;
+}
+
+template <typename XR>
+__device__ __forceinline__ int walk_terminal_plain(const XR& xrow, const DNode* __restrict__ nodes, int maxnode) {
+    int cur = 0;
+    for (int k = 0; k < maxnode; ++k) {
+        const DNode nd = load_node(nodes, cur);
+        if (node_status(nd.meta) == -1) return cur;
+        cur = step_plain(nd, xrow(node_var(nd.meta)));
+        if (cur < 0) return 0;
+    }
+    return 0;
+}
+
+template <typename XR>
+__device__ __forceinline__ int walk_predict_plain(const XR& xrow, int nclass, const DNode* __restrict__ nodes,
+                                                  const int32_t* __restrict__ nclass_of, int maxnode) {
+    int cur = 0;
+    for (int k = 0; k < maxnode; ++k) {
+        const DNode nd = load_node(nodes, cur);
+        if (node_status(nd.meta) == -1) {
+            const int c = __ldg(nclass_of + cur);
+            return (c >= 0 && c < nclass) ? c : 0;
+        }
+        cur = step_plain(nd, xrow(node_var(nd.meta)));
+        if (cur < 0) return 0;
+    }
+    return -1;
+}
+
+// int(v + 0.5) in FP64, truncated, as far as a category index needs it: 0
+// below 0.5 (and for NaN), exact up to 2^23, and at least 2^23 beyond.  v's
+// distance to the next lower whole number is exact in FP32, so no conversion
+// to FP64 and back is needed.
+__device__ __forceinline__ int round_category(float v) {
+    if (!(v >= 0.5f)) return 0;
+    const float w = floorf(v);
+    return __float2int_rz(w) + (__fsub_rn(v, w) >= 0.5f ? 1 : 0);
+}
+
 // predict_classification's walk: returns the voted class, or -1 for no vote
 // (loop bound reached).  Invalid paths vote for class 0.
-__device__ __forceinline__ int walk_predict(const float* __restrict__ xrow, int p, int nclass,
-                                            const DNode* __restrict__ nodes, const int32_t* __restrict__ nclass_of,
-                                            const int32_t* __restrict__ cat, const int32_t* __restrict__ cgl,
-                                            int maxcat, int maxnode) {
+template <typename XR>
+__device__ __forceinline__ int walk_predict(const XR& xrow, int p, int nclass, const DNode* __restrict__ nodes,
+                                            const int32_t* __restrict__ nclass_of, const int32_t* __restrict__ cat,
+                                            const int32_t* __restrict__ cgl, int maxcat, int maxnode) {
     int kt = 0;
     for (int k = 0; k < maxnode; ++k) {
         if (kt >= maxnode) return 0;
@@ -274,16 +349,13 @@ __device__ __forceinline__ int walk_predict(const float* __restrict__ xrow, int 
         }
         const int m = node_var(nd.meta);
         if (m >= p) return 0;
-        const float v = __ldg(xrow + m);
+        const float v = xrow(m);
         if (!node_cat(nd.meta)) {
             kt = (v <= nd.split) ? nd.left : nd.right;
         } else {
-            const int j = __double2int_rz(__dadd_rn((double)v, 0.5));
-            if (j >= 1 && j <= __ldg(cat + m)) {
-                kt = (cgl_at(cgl, maxcat, kt, j - 1) == 1) ? nd.left : nd.right;
-            } else {
-                return 0;
-            }
+            const int j = round_category(v);
+            if (j < 1 || j > __ldg(cat + m)) return 0;
+            kt = (cgl_at(cgl, maxcat, kt, j - 1) == 1) ? nd.left : nd.right;
         }
     }
     return -1;
