@@ -39,7 +39,7 @@ namespace rfx {
 
 namespace {
 
-constexpr int VT = 256;  // threads of the per-tree OOB-list kernel
+constexpr int VT = 512;  // threads of the per-tree OOB-list kernel
 
 enum { DIR_BREAK = -2 };
 
@@ -112,61 +112,60 @@ joob_kernel(const uint8_t* __restrict__ inbag, int n, int32_t* __restrict__ joob
             const int32_t* __restrict__ permoff, const int32_t* __restrict__ perm_all,
             int32_t* __restrict__ partner_all, const int32_t* __restrict__ memb = nullptr,
             int32_t* __restrict__ oobord = nullptr) {
-    __shared__ int wsum[VT / 32];
-    __shared__ int s_base;
+    __shared__ int wsum[2][VT / 32];
     const int t = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint8_t* ib = inbag + (size_t)t * n;
     int32_t* joob = joob_all + (size_t)t * n;
-    if (tid == 0) s_base = 0;
-    __syncthreads();
-    // JB consecutive samples per thread (their flag loads in flight
-    // together), JB * VT samples per round
-    constexpr int JB = 4;
-    for (int base = 0; base < n; base += JB * VT) {
-        const int i0 = base + JB * tid;
-        unsigned fl = 0;
-#pragma unroll
-        for (int u = 0; u < JB; ++u)
-            if (i0 + u < n && ib[i0 + u] == 0) fl |= 1u << u;
-        const int cnt = __popc(fl);
-        int incl = cnt;  // inclusive warp scan of the per-thread counts
+    // place of this thread's cnt entries after the `base` of earlier rounds,
+    // and base past this round's; one barrier a round (the warps' sums
+    // alternate between two rows)
+    int base = 0, buf = 0;
+    auto place = [&](int cnt) -> int {
+        int incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int v = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= d) incl += v;
         }
-        if (lane == 31) wsum[wid] = incl;
+        if (lane == 31) wsum[buf][wid] = incl;
         __syncthreads();
-        int woff = 0, tot = 0;
-        for (int q = 0; q < VT / 32; ++q) {
-            if (q < wid) woff += wsum[q];
-            tot += wsum[q];
-        }
-        int pos = s_base + woff + incl - cnt;
+        const int ws = lane < VT / 32 ? wsum[buf][lane] : 0;
+        const int woff = __reduce_add_sync(0xffffffffu, lane < wid ? ws : 0);
+        const int pos = base + woff + incl - cnt;
+        base += __reduce_add_sync(0xffffffffu, ws);
+        buf ^= 1;
+        return pos;
+    };
+    // JB consecutive samples per thread (their flag loads in flight
+    // together), JB * VT samples per round
+    constexpr int JB = 4;
+    for (int b0 = 0; b0 < n; b0 += JB * VT) {
+        const int i0 = b0 + JB * tid;
+        unsigned fl = 0;
+#pragma unroll
+        for (int u = 0; u < JB; ++u)
+            if (i0 + u < n && ib[i0 + u] == 0) fl |= 1u << u;
+        int pos = place(__popc(fl));
 #pragma unroll
         for (int u = 0; u < JB; ++u)
             if ((fl >> u) & 1u) joob[pos++] = i0 + u;
-        __syncthreads();
-        if (tid == 0) s_base += tot;
-        __syncthreads();
     }
     if (!partner_all) return;
     // the permutation partner of every OOB sample, indexed by sample:
     // partner[joob[r]] = joob[perm[r]] (cpu_permobmr's swap order)
-    const int noob = s_base;
+    const int noob = base;
     const int32_t* perm = perm_all + permoff[t];
     int32_t* partner = partner_all + (size_t)t * n;
+    __syncthreads();  // joob is complete
     for (int r = tid; r < noob; r += VT) partner[joob[r]] = joob[__ldg(perm + r)];
     if (!memb) return;
     // the OOB samples in member-list order (by leaf): the walk's thread order
     const int32_t* mt = memb + (size_t)t * n;
     int32_t* ord = oobord + (size_t)t * n;
-    __syncthreads();
-    if (tid == 0) s_base = 0;
-    __syncthreads();
-    for (int base = 0; base < n; base += JB * VT) {
-        const int q0 = base + JB * tid;
+    base = 0;
+    for (int b0 = 0; b0 < n; b0 += JB * VT) {
+        const int q0 = b0 + JB * tid;
         int mv[JB];
         unsigned fl = 0;
 #pragma unroll
@@ -174,27 +173,10 @@ joob_kernel(const uint8_t* __restrict__ inbag, int n, int32_t* __restrict__ joob
             mv[u] = q0 + u < n ? __ldg(mt + q0 + u) : 0;
             if (q0 + u < n && ib[mv[u]] == 0) fl |= 1u << u;
         }
-        const int cnt = __popc(fl);
-        int incl = cnt;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += v;
-        }
-        if (lane == 31) wsum[wid] = incl;
-        __syncthreads();
-        int woff = 0, tot = 0;
-        for (int q = 0; q < VT / 32; ++q) {
-            if (q < wid) woff += wsum[q];
-            tot += wsum[q];
-        }
-        int pos = s_base + woff + incl - cnt;
+        int pos = place(__popc(fl));
 #pragma unroll
         for (int u = 0; u < JB; ++u)
             if ((fl >> u) & 1u) ord[pos++] = mv[u];
-        __syncthreads();
-        if (tid == 0) s_base += tot;
-        __syncthreads();
     }
 }
 
@@ -630,20 +612,21 @@ __global__ void varimp_feature_kernel(const int32_t* __restrict__ counts, const 
     const int lane = threadIdx.x & 31;
     if (k >= p) return;
     float a = 0.0f, s = 0.0f;
+    // rr of tree t (0 where the tree does not use the feature); the next 32
+    // trees' are formed with the current ones' sums
+    auto rr_of = [&](int t, bool& used) -> float {
+        used = t < T && ((__ldg(iv + (size_t)min(t, T - 1) * W + (k >> 6)) >> (k & 63)) & 1ull);
+        if (!used) return 0.0f;
+        const int right = __ldg(counts + 2 * t), rightimp = __ldg(counts + 2 * t + 1) + __ldg(delta + (size_t)t * p + k);
+        return __fdiv_rn(__fsub_rn((float)right, (float)rightimp), (float)__ldg(noob + t));
+    };
+    bool nused;
+    float nrr = rr_of(lane, nused);
     for (int t0 = 0; t0 < T; t0 += 32) {
-        const int t = t0 + lane;
-        bool used = false;
-        float rr = 0.0f, r2 = 0.0f;
-        if (t < T) {
-            used = (iv[(size_t)t * W + (k >> 6)] >> (k & 63)) & 1ull;
-            if (used) {
-                const int rightimp = counts[2 * t + 1] + delta[(size_t)t * p + k];
-                rr = __fdiv_rn(__fsub_rn((float)counts[2 * t], (float)rightimp), (float)noob[t]);
-                r2 = __fmul_rn(rr, rr);
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, used);
-#pragma unroll 8
+        const float rr = nrr, r2 = __fmul_rn(nrr, nrr);
+        const unsigned m = __ballot_sync(0xffffffffu, nused);
+        nrr = rr_of(t0 + 32 + lane, nused);
+#pragma unroll
         for (int l = 0; l < 32; ++l) {
             const float x = __shfl_sync(0xffffffffu, rr, l);
             const float x2 = __shfl_sync(0xffffffffu, r2, l);
