@@ -22,8 +22,6 @@ int grow_forest(const float* X, const int32_t* y, int n, int p, int nclass, int 
 
 namespace rfx {
 
-rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf);
-
 namespace {
 thread_local std::string g_last_error;
 
@@ -200,7 +198,6 @@ static rfx_status with_f64_out(Ctx* c, double* out, size_t len, const char* who,
         st = copy_out(c, out, d, sizeof(double) * len);
         if (st == RFX_OK) st = finish_host(c, true);
     }
-    cudaStreamSynchronize(c->stream);
     return st;
 }
 
@@ -245,6 +242,7 @@ rfx_status rfx_ctx_create(const rfx_config* cfg, rfx_ctx** out) {
         return st;
     }
     cudaMemset(c->d_err, 0, sizeof(uint32_t));
+    cudaMemset(c->d_pairs, 0, 4 * sizeof(unsigned long long));
     *out = reinterpret_cast<rfx_ctx*>(c);
     return RFX_OK;
 }
@@ -647,6 +645,10 @@ rfx_status rfx_route_oob(rfx_ctx* ctx, int32_t* q, int32_t* nout, int32_t* leaf)
         set_error("rfx_route_oob: a case-wise context weighs the votes (float): use rfx_casewise_votes");
         return RFX_ERR_STATE;
     }
+    // device outputs are written by the routing itself, host ones copied out
+    const bool qdev = is_device_ptr(q), ndev = is_device_ptr(nout);
+    int32_t* dq = qdev ? q : nullptr;
+    int32_t* dn = ndev ? nout : nullptr;
     bool any_host = false;
     if (leaf) {
         int32_t* dleaf = leaf;
@@ -655,23 +657,23 @@ rfx_status rfx_route_oob(rfx_ctx* ctx, int32_t* q, int32_t* nout, int32_t* leaf)
             if ((st = dalloc(c, &c->d_joob, (size_t)c->T * c->n))) return st;  // reuse as staging
             dleaf = c->d_joob;
         }
-        if ((st = launch_route_leaf(c, dleaf))) return st;
+        if ((st = launch_route_leaf(c, dleaf, dq, dn))) return st;
         RFX_CUDA(cudaGetLastError());
         if (!dev) {
             if ((st = copy_out(c, leaf, dleaf, sizeof(int32_t) * (size_t)c->T * c->n))) return st;
             any_host = true;
         }
-    } else if ((st = launch_route(c))) {
+    } else if ((st = launch_route(c, dq, dn))) {
         return st;
     }
     c->routed = true;
     c->csr_built = false;
-    if (q) {
-        any_host |= !is_device_ptr(q);
+    if (q && !qdev) {
+        any_host = true;
         if ((st = copy_out(c, q, c->d_votes, sizeof(int32_t) * (size_t)c->n * c->nclass))) return st;
     }
-    if (nout) {
-        any_host |= !is_device_ptr(nout);
+    if (nout && !ndev) {
+        any_host = true;
         if ((st = copy_out(c, nout, c->d_nout, sizeof(int32_t) * (size_t)c->n))) return st;
     }
     return finish_host(c, any_host);
@@ -716,7 +718,6 @@ rfx_status rfx_oob_summary(rfx_ctx* ctx, float* oob_error, int32_t* pred, float*
         if (!dq) st = RFX_ERR_OOM;
         if (st == RFX_OK) st = casewise_votes_into(c, dq);
         if (st == RFX_OK) st = launch_oob_summary_f32(c, dq, d_e, d_p, d_pr);
-        if (st == RFX_OK) cudaStreamSynchronize(c->stream);
     } else {
         st = launch_oob_summary(c, d_e, d_p, d_pr);
     }
@@ -724,7 +725,7 @@ rfx_status rfx_oob_summary(rfx_ctx* ctx, float* oob_error, int32_t* pred, float*
     if (st == RFX_OK && hp) st = copy_out(c, pred, d_p, sizeof(int32_t) * c->n);
     if (st == RFX_OK && hpr) st = copy_out(c, proba, d_pr, sizeof(float) * (size_t)c->n * c->nclass);
     if (st == RFX_OK) st = finish_host(c, he || hp || hpr);
-    cudaStreamSynchronize(c->stream);
+    if (!tmp.empty()) cudaStreamSynchronize(c->stream);
     for (void* d : tmp) cudaFree(d);
     return st;
 }
@@ -781,8 +782,8 @@ static rfx_status casewise_votes_into(Ctx* c, float* dq) {
         c->csr_built = false;
         st = launch_tnodewt(c);
     }
+    // (the scratch goes back to the pool, where only later work of this stream takes it)
     if (st == RFX_OK) st = launch_casewise_votes(c, dleaf, dq);
-    if (st == RFX_OK) RFX_CUDA(cudaStreamSynchronize(c->stream));  // the scratch goes back to the pool
     return st;
 }
 
@@ -813,9 +814,7 @@ rfx_status rfx_casewise_votes(rfx_ctx* ctx, float* q, int32_t* nout) {
         any_host |= !is_device_ptr(nout);
         if ((st = copy_out(c, nout, c->d_nout, sizeof(int32_t) * (size_t)c->n))) return st;
     }
-    st = finish_host(c, any_host);
-    cudaStreamSynchronize(c->stream);
-    return st;
+    return finish_host(c, any_host);
 }
 
 rfx_status rfx_proximity_upper_f64(rfx_ctx* ctx, double* S, size_t len) {
@@ -906,9 +905,7 @@ rfx_status rfx_proximity_rfgap(rfx_ctx* ctx, double* P, size_t len) {
                                       c->d_err)))
             return s;
         StageTimer stt(c, ST_PAIRS, 0);
-        s = launch_weighted_rows(c, 1, key, dsb, segoff, memb, sb[T], dP);
-        if (s == RFX_OK) RFX_CUDA(cudaStreamSynchronize(c->stream));  // the scratch goes back to the pool
-        return s;
+        return launch_weighted_rows(c, 1, key, dsb, segoff, memb, sb[T], dP);
     });
 }
 

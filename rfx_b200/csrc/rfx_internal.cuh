@@ -275,7 +275,7 @@ rfx_status allow_dyn_smem(K* kernel, int dev_smem) {
 }
 
 // kernel launchers (each returns after enqueueing on ctx->stream)
-rfx_status launch_route(Ctx* c);
+rfx_status launch_route(Ctx* c, int32_t* votes_out = nullptr, int32_t* nout_out = nullptr);
 rfx_status launch_build_csr(Ctx* c);
 
 // Autotuned stages: kernel ids and the launch shapes each offers.
@@ -303,7 +303,7 @@ rfx_status launch_weighted_rows(Ctx* c, int mode, const int32_t* key, const int6
 rfx_status launch_gap_keys(Ctx* c, const int32_t* d_leafnode, int32_t* d_key);
 rfx_status launch_casewise_varimp(Ctx* c, const int32_t* d_leafnode, int impn, float* d_avimp, float* d_sqsd,
                                   float* d_qimp, float* d_qimpm);
-rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf);
+rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf, int32_t* votes_out = nullptr, int32_t* nout_out = nullptr);
 rfx_status launch_oob_summary_f32(Ctx* c, const float* d_q, float* d_errout, int32_t* d_pred, float* d_proba);
 rfx_status launch_finishprox_f64(Ctx* c, const double* dS, float* dP, int full);
 // S_hub tiles of the hub leaves (hubs.cu)

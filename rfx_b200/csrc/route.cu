@@ -384,10 +384,14 @@ void route_launch(Ctx* c, int shape, int32_t* d_leaf) {
 // nout[i] = 2 * (number of trees with i out of bag): the reference increments
 // it in cpu_bootstrap and again in the vote loop.  32 samples per CTA, the
 // trees dealt over its warps (one thread per sample waited for T loads in a
-// few long chains: 51 us at n = 50,000 / 1,000 trees, 30 us this way).
+// few long chains: 51 us at n = 50,000 / 1,000 trees, 30 us this way).  Runs
+// after the walks: it also copies the finished votes and its counts to the
+// caller's device buffers (either may be null).
 constexpr int NOUT_WARPS = 16;
 __global__ void __launch_bounds__(NOUT_WARPS * 32)
-nout_kernel(const uint8_t* __restrict__ inbag, int n, int T, int32_t* __restrict__ nout) {
+nout_kernel(const uint8_t* __restrict__ inbag, int n, int T, int32_t* __restrict__ nout,
+            const int32_t* __restrict__ votes, int nclass, int32_t* __restrict__ votes_out,
+            int32_t* __restrict__ nout_out) {
     __shared__ int s_c[NOUT_WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
@@ -403,47 +407,61 @@ nout_kernel(const uint8_t* __restrict__ inbag, int n, int T, int32_t* __restrict
 #pragma unroll
         for (int q = 0; q < NOUT_WARPS; ++q) sum += s_c[q][lane];
         nout[i] = 2 * sum;
+        if (nout_out) nout_out[i] = 2 * sum;
+    }
+    if (votes_out) {
+        const size_t v0 = (size_t)blockIdx.x * 32 * nclass, v1 = min((size_t)n * nclass, v0 + 32 * (size_t)nclass);
+        for (size_t e = v0 + threadIdx.x; e < v1; e += NOUT_WARPS * 32) votes_out[e] = votes[e];
     }
 }
 
 // OOB error / prediction / probability from integer votes, with the
 // reference's float arithmetic: argmax with >= (ties to the higher class),
 // total votes summed in float, probability = q / total (or 1/nclass).
+// The CTAs add their counts to counts[0..1]; the last one to finish (ticket
+// counts[2]) forms the error and leaves the three words zero for the next call.
+// One launch instead of a clear and two kernels.
 template <typename TV>
-__global__ void oob_summary_kernel(const TV* __restrict__ votes, const int32_t* __restrict__ nout,
-                                   const int32_t* __restrict__ y, int n, int nclass, int32_t* __restrict__ pred,
-                                   float* __restrict__ proba, unsigned int* __restrict__ counts) {
+__global__ void __launch_bounds__(256)
+oob_summary_kernel(const TV* __restrict__ votes, const int32_t* __restrict__ nout, const int32_t* __restrict__ y,
+                   int n, int nclass, int32_t* __restrict__ pred, float* __restrict__ proba,
+                   unsigned int* __restrict__ counts, float* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const TV* q = votes + (size_t)i * nclass;
-    const float uni = __double2float_rn(1.0 / (double)nclass);
-    if (nout[i] > 0) {
+    bool some = false, right = false;
+    if (i < n) {
+        const TV* q = votes + (size_t)i * nclass;
+        const float uni = __double2float_rn(1.0 / (double)nclass);
         int best = 0;
-        float mx = (float)q[0];
-        float tot = 0.0f;
-        for (int c = 0; c < nclass; ++c) {
-            const float v = (float)q[c];
-            tot = __fadd_rn(tot, v);
-            if (v >= mx) {
-                mx = v;
-                best = c;
+        if (nout[i] > 0) {
+            float mx = (float)q[0];
+            float tot = 0.0f;
+            for (int c = 0; c < nclass; ++c) {
+                const float v = (float)q[c];
+                tot = __fadd_rn(tot, v);
+                if (v >= mx) {
+                    mx = v;
+                    best = c;
+                }
             }
+            if (proba)
+                for (int c = 0; c < nclass; ++c)
+                    proba[(size_t)i * nclass + c] = tot > 0.0f ? __fdiv_rn((float)q[c], tot) : uni;
+            some = true;
+            right = best == y[i];
+        } else if (proba) {
+            for (int c = 0; c < nclass; ++c) proba[(size_t)i * nclass + c] = uni;
         }
         if (pred) pred[i] = best;
-        if (proba)
-            for (int c = 0; c < nclass; ++c)
-                proba[(size_t)i * nclass + c] = tot > 0.0f ? __fdiv_rn((float)q[c], tot) : uni;
-        atomicAdd(counts + 0, 1u);
-        if (best == y[i]) atomicAdd(counts + 1, 1u);
-    } else {
-        if (pred) pred[i] = 0;
-        if (proba)
-            for (int c = 0; c < nclass; ++c) proba[(size_t)i * nclass + c] = uni;
     }
-}
-
-__global__ void oob_error_kernel(const unsigned int* __restrict__ counts, float* __restrict__ err) {
-    const unsigned total = counts[0], correct = counts[1];
+    const unsigned ns = __syncthreads_count(some), nr = __syncthreads_count(right);
+    if (!err || threadIdx.x != 0) return;
+    if (ns) atomicAdd(counts, ns);
+    if (nr) atomicAdd(counts + 1, nr);
+    __threadfence();
+    if (atomicAdd(counts + 2, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const unsigned total = atomicExch(counts, 0u), correct = atomicExch(counts + 1, 0u);
+    counts[2] = 0u;
     *err = total > 0 ? __fsub_rn(1.0f, __fdiv_rn((float)correct, (float)total)) : 0.0f;
 }
 
@@ -526,13 +544,16 @@ transpose_kernel(const float* __restrict__ X, int m, int p, int ms, float* __res
 
 }  // namespace
 
-static rfx_status launch_nout(Ctx* c) {
-    nout_kernel<<<(c->n + 31) / 32, NOUT_WARPS * 32, 0, c->stream>>>(c->d_inbag, c->n, c->T, c->d_nout);
+static rfx_status launch_nout(Ctx* c, int32_t* votes_out, int32_t* nout_out) {
+    nout_kernel<<<(c->n + 31) / 32, NOUT_WARPS * 32, 0, c->stream>>>(c->d_inbag, c->n, c->T, c->d_nout, c->d_votes,
+                                                                     c->nclass, votes_out, nout_out);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }
 
-rfx_status launch_route(Ctx* c) {
+// Routing, votes and nout; the votes and nout also go to the given device
+// buffers (null: none).
+rfx_status launch_route(Ctx* c, int32_t* votes_out, int32_t* nout_out) {
     StageTimer st(c, ST_ROUTE, 2);
     rfx_status r;
     if (c->csr_built) {
@@ -591,45 +612,35 @@ rfx_status launch_route(Ctx* c) {
         });
     }
     if (r != RFX_OK) return r;
-    return launch_nout(c);
+    return launch_nout(c, votes_out, nout_out);
 }
 
 // launch_route with the node ids written as well.
-rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf) {
+rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf, int32_t* votes_out, int32_t* nout_out) {
     StageTimer st(c, ST_ROUTE, 2);
     RFX_CUDA(cudaMemsetAsync(c->d_votes, 0, sizeof(int32_t) * (size_t)c->n * c->nclass, c->stream));
     route_launch(c, 0, d_leaf);
     RFX_CUDA(cudaGetLastError());
-    return launch_nout(c);
+    return launch_nout(c, votes_out, nout_out);
+}
+
+template <typename TV>
+static rfx_status oob_summary(Ctx* c, const TV* votes, float* d_errout, int32_t* d_pred, float* d_proba) {
+    StageTimer st(c, ST_OOB, 1);
+    unsigned int* counts = reinterpret_cast<unsigned int*>(c->d_pairs) + 2;  // scratch words after the pair counter
+    oob_summary_kernel<TV><<<(c->n + 255) / 256, 256, 0, c->stream>>>(votes, c->d_nout, c->d_y, c->n, c->nclass,
+                                                                      d_pred, d_proba, counts, d_errout);
+    RFX_CUDA(cudaGetLastError());
+    return RFX_OK;
 }
 
 rfx_status launch_oob_summary(Ctx* c, float* d_errout, int32_t* d_pred, float* d_proba) {
-    StageTimer st(c, ST_OOB, d_errout ? 2 : 1);
-    unsigned int* counts = reinterpret_cast<unsigned int*>(c->d_pairs) + 2;  // scratch words after the pair counter
-    RFX_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned int), c->stream));
-    oob_summary_kernel<int32_t><<<(c->n + 255) / 256, 256, 0, c->stream>>>(c->d_votes, c->d_nout, c->d_y, c->n,
-                                                                            c->nclass, d_pred, d_proba, counts);
-    RFX_CUDA(cudaGetLastError());
-    if (d_errout) {
-        oob_error_kernel<<<1, 1, 0, c->stream>>>(counts, d_errout);
-        RFX_CUDA(cudaGetLastError());
-    }
-    return RFX_OK;
+    return oob_summary<int32_t>(c, c->d_votes, d_errout, d_pred, d_proba);
 }
 
 // the same from float votes (case-wise weights)
 rfx_status launch_oob_summary_f32(Ctx* c, const float* d_q, float* d_errout, int32_t* d_pred, float* d_proba) {
-    StageTimer st(c, ST_OOB, d_errout ? 2 : 1);
-    unsigned int* counts = reinterpret_cast<unsigned int*>(c->d_pairs) + 2;  // scratch words after the pair counter
-    RFX_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned int), c->stream));
-    oob_summary_kernel<float><<<(c->n + 255) / 256, 256, 0, c->stream>>>(d_q, c->d_nout, c->d_y, c->n,
-                                                                            c->nclass, d_pred, d_proba, counts);
-    RFX_CUDA(cudaGetLastError());
-    if (d_errout) {
-        oob_error_kernel<<<1, 1, 0, c->stream>>>(counts, d_errout);
-        RFX_CUDA(cudaGetLastError());
-    }
-    return RFX_OK;
+    return oob_summary<float>(c, d_q, d_errout, d_pred, d_proba);
 }
 
 rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
