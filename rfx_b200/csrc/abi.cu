@@ -400,6 +400,12 @@ static rfx_status load_forest(Ctx* c, const LoadInput& in) {
         st = launch_pack_forest(s, T, n, p, c->d_offs, r_status, r_bestvar, r_split, r_treemap, c->d_cat, r_nin,
                                 c->d_nodes, c->d_leafidx, c->d_iv, r_nleaf, c->d_inbag, c->d_noob, r_err);
         c->launches += 2;
+        bool levels = false;
+        for (int m = 0; m < p; ++m) levels |= in.cat[m] != 1;
+        if (st == RFX_OK && levels) {
+            st = launch_level_check(s, c->d_X, n, p, c->d_cat, maxcat, r_err);
+            c->launches += 1;
+        }
         LoadError herr{};
         if (st == RFX_OK) {
             e = cudaMemcpyAsync(nleaf.data(), r_nleaf, sizeof(int32_t) * T, cudaMemcpyDeviceToHost, s);
@@ -494,6 +500,7 @@ static rfx_status load_forest(Ctx* c, const LoadInput& in) {
         int most_levels = 0;
         for (int m = 0; m < p; ++m) most_levels = std::max(most_levels, in.cat[m]);
         c->plain_walks = !in.has_catgoleft && most_levels <= (1 << 20) && c->max_nnode <= 2 * n + 1;
+        c->plain_imp = !in.has_catgoleft && !herr.off_level;
         ALLOC(d_segoff, segbase[T]);
 #undef ALLOC
         if (st != RFX_OK) {

@@ -89,6 +89,20 @@ pack_nodes_kernel(const int64_t* __restrict__ offs, const int32_t* __restrict__ 
     if (tid == 0) nleaf[t] = base;
 }
 
+// Whether a categorical value of the training rows rounds (cpu_testreeimp's
+// rule, float x + 0.5 truncated) outside 0..maxcat-1.
+__global__ void __launch_bounds__(LD_THREADS)
+level_check_kernel(const float* __restrict__ X, size_t count, int p, const int32_t* __restrict__ cat, int maxcat,
+                   LoadError* __restrict__ err) {
+    bool off = false;
+    for (size_t e = (size_t)blockIdx.x * LD_THREADS + threadIdx.x; e < count; e += (size_t)gridDim.x * LD_THREADS) {
+        if (__ldg(cat + e % p) == 1) continue;
+        const int j = __float2int_rz(__fadd_rn(__ldg(X + e), 0.5f));
+        off |= j < 0 || j >= maxcat;
+    }
+    if (off) err->off_level = 1;
+}
+
 // Per tree: bag flags (nin > 0) and the OOB count; negative multiplicities fail.
 __global__ void __launch_bounds__(LD_THREADS)
 bag_kernel(const int32_t* __restrict__ nin, int n, uint8_t* __restrict__ inbag, int32_t* __restrict__ noob,
@@ -151,6 +165,16 @@ cudaError_t launch_gather_padded(cudaStream_t s, int T, int maxnode, int maxcat,
                                                   nodeclass_p, catgoleft_p, status, bestvar, split, treemap, nodeclass,
                                                   catgoleft);
     return cudaGetLastError();
+}
+
+rfx_status launch_level_check(cudaStream_t s, const float* X, int n, int p, const int32_t* d_cat, int maxcat,
+                              LoadError* err) {
+    const size_t count = (size_t)n * p;
+    const size_t blocks = (count + LD_THREADS - 1) / LD_THREADS;
+    level_check_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), LD_THREADS, 0, s>>>(X, count, p, d_cat, maxcat,
+                                                                                        err);
+    RFX_CUDA(cudaGetLastError());
+    return RFX_OK;
 }
 
 rfx_status launch_pack_forest(cudaStream_t s, int T, int n, int p, const int64_t* d_offs, const int32_t* status,

@@ -67,6 +67,7 @@ struct Ctx {
     int max_nnode = 0;
     int iv_words = 0;                   // ceil(p / 64)
     bool plain_walks = false;           // see walk_terminal_plain (walks.cuh)
+    bool plain_imp = false;             // and every categorical training value rounds to 0..maxcat-1
 
     float* d_X = nullptr;               // n*p
     int32_t* d_y = nullptr;             // n
@@ -159,7 +160,7 @@ struct LoadError {
     int code;  // 1 nodestatus, 2 bestvar, 3 child, 4 negative nin
     int tree;
     int node;  // node within the tree, or sample for code 4
-    int pad;
+    int off_level;  // (not a failure) a categorical training value rounds outside 0..maxcat-1
 };
 
 // Per-call scratch drawn from the context's pool: get() reuses a kept block of
@@ -286,6 +287,8 @@ rfx_status launch_pack_forest(cudaStream_t s, int T, int n, int p, const int64_t
                               const int32_t* bestvar, const float* split, const int32_t* treemap,
                               const int32_t* d_cat, const int32_t* nin, DNode* nodes, int32_t* leafidx,
                               uint64_t* iv, int32_t* nleaf, uint8_t* inbag, int32_t* noob, LoadError* err);
+rfx_status launch_level_check(cudaStream_t s, const float* X, int n, int p, const int32_t* d_cat, int maxcat,
+                              LoadError* err);
 cudaError_t launch_gather_padded(cudaStream_t s, int T, int maxnode, int maxcat, const int64_t* d_offs,
                                  const int32_t* status_p, const int32_t* bestvar_p, const float* split_p,
                                  const int32_t* treemap_p, const int32_t* nodeclass_p, const int32_t* catgoleft_p,
