@@ -12,7 +12,7 @@ namespace rfx {
 // (a loop of one load and one add waits for each).
 constexpr int SUM_BATCH = 20;
 template <typename T>
-__device__ __forceinline__ T warp_part_sum(const T* __restrict__ part, int nparts, size_t stride, int lane) {
+__device__ __forceinline__ T warp_part_sum(const T* part, int nparts, size_t stride, int lane) {
     T v = 0;
     for (int q0 = lane; q0 < nparts; q0 += 32 * SUM_BATCH) {
         T x[SUM_BATCH];

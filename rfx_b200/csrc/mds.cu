@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "dense.cuh"
+#include "pdl.cuh"
 #include "rfx_internal.cuh"
 
 namespace rfx {
@@ -184,9 +185,10 @@ __device__ __forceinline__ size_t frag_pos(int k, int c) {
     return (size_t)(k >> 2) * 64 + (c >> 3) * 32 + (c & 7) * 4 + (k & 3);
 }
 
-__global__ void __launch_bounds__(128, 1) dgemm_bv_kernel(const double* __restrict__ B, int nt,
-                                                         const double* __restrict__ Vf, int n, int kchunk,
-                                                         double* __restrict__ Wpart, uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(128, 1) dgemm_bv_kernel(const double* B, int nt,
+                                                         const double* Vf, int n, int kchunk,
+                                                         double* Wpart, uint32_t* err) {
+    pdl_begin();
     extern __shared__ __align__(128) uint8_t dsm[];
     __shared__ __align__(8) uint64_t full[DB_STAGES];
     __shared__ int s_fail;
@@ -269,7 +271,8 @@ __global__ void __launch_bounds__(128, 1) dgemm_bv_kernel(const double* __restri
 }
 
 // W = sum of the ksn partial products, added in range order (reproducible).
-__global__ void bv_reduce_kernel(const double* __restrict__ Wpart, int n, int ksn, double* __restrict__ W) {
+__global__ void bv_reduce_kernel(const double* Wpart, int n, int ksn, double* W) {
+    pdl_begin();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t cnt = (size_t)n * S_BLK;
     if (idx >= cnt) return;
@@ -281,8 +284,9 @@ __global__ void bv_reduce_kernel(const double* __restrict__ Wpart, int n, int ks
 // G[S x S] += X^T Y over rows (atomics into a zeroed G).
 // Per-CTA partial Gram matrices X^T Y (16 x 16) into part[blockIdx.x], added
 // by gram_sum_kernel in a fixed order (reproducible run to run).
-__global__ void __launch_bounds__(256) dgram_kernel(const double* __restrict__ X, const double* __restrict__ Y, int n,
-                                                    double* __restrict__ part) {
+__global__ void __launch_bounds__(256) dgram_kernel(const double* X, const double* Y, int n,
+                                                    double* part) {
+    pdl_begin();
     __shared__ double Xs[64][S_BLK], Ys[64][S_BLK];
     const int tid = threadIdx.x;
     const int a = tid / S_BLK, b = tid % S_BLK;  // 16 x 16 outputs
@@ -302,7 +306,8 @@ __global__ void __launch_bounds__(256) dgram_kernel(const double* __restrict__ X
 
 // G[e] = sum over the partials, one warp per entry (lane l the partials l,
 // l + 32, ..., then a fixed shuffle tree)
-__global__ void gram_sum_kernel(const double* __restrict__ part, int nparts, double* __restrict__ G) {
+__global__ void gram_sum_kernel(const double* part, int nparts, double* G) {
+    pdl_begin();
     const int e = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (e >= S_BLK * S_BLK) return;
@@ -318,7 +323,7 @@ constexpr int SMALL_THREADS = 512;
 
 // The 16 x 16 matrix into shared memory (leading dim ld): from G, or summed
 // from nparts <= GRAM_FUSE partials (a warp takes every 16th entry).
-__device__ __forceinline__ void load_gram(const double* __restrict__ G, const double* __restrict__ part, int nparts,
+__device__ __forceinline__ void load_gram(const double* G, const double* part, int nparts,
                                           double* out, int ld) {
     if (!part) {
         for (int e = threadIdx.x; e < S_BLK * S_BLK; e += SMALL_THREADS) out[(e / S_BLK) * ld + e % S_BLK] = G[e];
@@ -342,9 +347,10 @@ __device__ __forceinline__ void load_gram(const double* __restrict__ G, const do
 // A serial chain (16 square roots and divisions): 9.5 us from G, 15 us with
 // the sum of 32 partials (18 us, and 2 for the sum's own launch, with a dot
 // product per entry in one thread's chain).
-__global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* __restrict__ G,
-                                                                 const double* __restrict__ part, int nparts,
-                                                                 double* __restrict__ Tm, int* __restrict__ bad) {
+__global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* G,
+                                                                 const double* part, int nparts,
+                                                                 double* Tm, int* bad) {
+    pdl_begin();
     __shared__ double L[S_BLK * S_BLK], Li[S_BLK * S_BLK];
     __shared__ double flag;
     load_gram(G, part, nparts, L, S_BLK);
@@ -358,8 +364,9 @@ __global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* _
 
 // V = W T (rows of W times an S x S matrix), and with Vf the same in fragment
 // order for the next product.
-__global__ void dright_kernel(const double* __restrict__ W, const double* __restrict__ Tm, int n,
-                              double* __restrict__ V, double* __restrict__ Vf) {
+__global__ void dright_kernel(const double* W, const double* Tm, int n,
+                              double* V, double* Vf) {
+    pdl_begin();
     __shared__ double Ts[S_BLK * S_BLK];
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) Ts[e] = Tm[e];
     __syncthreads();
@@ -370,7 +377,7 @@ __global__ void dright_kernel(const double* __restrict__ W, const double* __rest
     const double2* wr = reinterpret_cast<const double2*>(W + (size_t)r * S_BLK);
 #pragma unroll
     for (int k = 0; k < S_BLK / 2; ++k) {
-        const double2 x = __ldg(wr + k);
+        const double2 x = *(wr + k);
         w[2 * k] = x.x;
         w[2 * k + 1] = x.y;
     }
@@ -382,9 +389,10 @@ __global__ void dright_kernel(const double* __restrict__ W, const double* __rest
 }
 
 // One CTA: eigen-decomposition of the S x S projection H (symmetrised).
-__global__ void __launch_bounds__(SMALL_THREADS) rr_kernel(const double* __restrict__ H,
-                                                           const double* __restrict__ part, int nparts,
-                                                           double* __restrict__ evals, double* __restrict__ evecs) {
+__global__ void __launch_bounds__(SMALL_THREADS) rr_kernel(const double* H,
+                                                           const double* part, int nparts,
+                                                           double* evals, double* evecs) {
+    pdl_begin();
     constexpr int LD = S_BLK + 1;
     __shared__ double Hs[S_BLK * S_BLK], A[S_BLK * LD], U[S_BLK * LD];
     __shared__ int pairs[2 * 64];
@@ -428,9 +436,10 @@ __device__ __forceinline__ uint64_t start_mix(uint64_t z) {
 // products in range order (ksn = 1: a plain block); out is also written in
 // fragment order for the next product (Vf), so a filter step is two launches,
 // the product and this.
-__global__ void block_axpby_kernel(double a, const double* __restrict__ X, int ksn, double b,
-                                   const double* __restrict__ Y, double c, const double* __restrict__ Z,
-                                   int64_t count, double* __restrict__ out, double* __restrict__ Vf) {
+__global__ void block_axpby_kernel(double a, const double* X, int ksn, double b,
+                                   const double* Y, double c, const double* Z,
+                                   int64_t count, double* out, double* Vf) {
+    pdl_begin();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
     double x = X[e];
@@ -503,19 +512,19 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
     // that reads it adds the few there are
     const double* fuse = gb <= GRAM_FUSE ? gpart : nullptr;
     auto gram = [&](const double* X, const double* Y) {
-        dgram_kernel<<<gb, 256, 0, s>>>(X, Y, n, gpart);
-        if (!fuse) gram_sum_kernel<<<S_BLK * S_BLK * 32 / 256, 256, 0, s>>>(gpart, gb, G);
+        launch_next(dgram_kernel, gb, 256, 0, s, X, Y, n, gpart);
+        if (!fuse) launch_next(gram_sum_kernel, S_BLK * S_BLK * 32 / 256, 256, 0, s, gpart, gb, G);
         c->launches += fuse ? 1 : 2;
     };
     // CholeskyQR2: Out = (src L1^{-T}) L2^{-T}, through the temporary Xt
     auto orth = [&](const double* src, double* Out) -> rfx_status {
         const unsigned gr = (unsigned)(((size_t)n * S_BLK + 255) / 256);
         gram(src, src);
-        chol_inv_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, Tm, bad);
-        dright_kernel<<<gr, 256, 0, s>>>(src, Tm, n, Xt, nullptr);
+        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, Tm, bad);
+        launch_next(dright_kernel, gr, 256, 0, s, src, Tm, n, Xt, nullptr);
         gram(Xt, Xt);
-        chol_inv_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, Tm, bad);
-        dright_kernel<<<gr, 256, 0, s>>>(Xt, Tm, n, Out, Vf);
+        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, Tm, bad);
+        launch_next(dright_kernel, gr, 256, 0, s, Xt, Tm, n, Out, Vf);
         c->launches += 4;
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
@@ -528,7 +537,7 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
     // the k largest against the previous check into *delta
     auto ritz = [&](double* delta) -> rfx_status {
         gram(V, W);
-        rr_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, ev, U);
+        launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, ev, U);
         c->launches += 1;
         RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
         RFX_CUDA(cudaStreamSynchronize(s));
@@ -589,13 +598,13 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
             if (!(ee > 0.0)) break;
             // Y0 = V, Y1 = (B V - cc V) / ee, Y_{j+1} = 2 (B Y_j - cc Y_j) / ee - Y_{j-1}
             // (the first step reads V itself as Y0)
-            block_axpby_kernel<<<cb, 256, 0, s>>>(1.0 / ee, W, 1, -cc / ee, V, 0.0, nullptr, cnt, Y1, Vf);
+            launch_next(block_axpby_kernel, cb, 256, 0, s, 1.0 / ee, W, 1, -cc / ee, V, 0.0, nullptr, cnt, Y1, Vf);
             c->launches += 1;
             const double* before = V;
             for (int j = 2; j <= cheb; ++j) {
                 if ((st = apply(Y1, nullptr)) != RFX_OK) return st;
                 ++matvecs;
-                block_axpby_kernel<<<cb, 256, 0, s>>>(2.0 / ee, Wpart, ksn, -2.0 * cc / ee, Y1, -1.0, before, cnt, Y2,
+                launch_next(block_axpby_kernel, cb, 256, 0, s, 2.0 / ee, Wpart, ksn, -2.0 * cc / ee, Y1, -1.0, before, cnt, Y2,
                                                       Vf);
                 c->launches += 1;
                 before = Y1;
@@ -612,7 +621,7 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
         if (check) {
             // Rayleigh-Ritz on span(V): H = V^T (B V)
             gram(V, W);
-            rr_kernel<<<1, SMALL_THREADS, 0, s>>>(G, fuse, gb, ev, U);
+            launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, ev, U);
             c->launches += 1;
             RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
             RFX_CUDA(cudaStreamSynchronize(s));
@@ -693,7 +702,8 @@ constexpr int RED_CTAS = 1184;  // eight CTAs per SM
 
 // out[e] = scale * sum over p of part[p * cnt + e], one warp per e
 template <typename TV>
-__global__ void part_sum_kernel(const TV* __restrict__ part, int nparts, int cnt, TV scale, TV* __restrict__ out) {
+__global__ void part_sum_kernel(const TV* part, int nparts, int cnt, TV scale, TV* out) {
+    pdl_begin();
     const int e = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (e >= cnt) return;
@@ -701,8 +711,9 @@ __global__ void part_sum_kernel(const TV* __restrict__ part, int nparts, int cnt
     if (lane == 0) out[e] = s * scale;
 }
 
-__global__ void __launch_bounds__(256) colsum_part_kernel(const double* __restrict__ V, int n,
-                                                          double* __restrict__ part) {
+__global__ void __launch_bounds__(256) colsum_part_kernel(const double* V, int n,
+                                                          double* part) {
+    pdl_begin();
     const int r = threadIdx.x / S_BLK, j = threadIdx.x % S_BLK;  // 16 rows x 16 columns per pass
     double s = 0.0;
     for (int i = blockIdx.x * 16 + r; i < n; i += gridDim.x * 16) s += V[(size_t)i * S_BLK + j];
@@ -717,8 +728,9 @@ __global__ void __launch_bounds__(256) colsum_part_kernel(const double* __restri
 }
 
 // u = V - mean (FP64), also as FP32
-__global__ void center_kernel(const double* __restrict__ V, const double* __restrict__ mean, int n,
-                              double* __restrict__ u, float* __restrict__ u32) {
+__global__ void center_kernel(const double* V, const double* mean, int n,
+                              double* u, float* u32) {
+    pdl_begin();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)n * S_BLK) return;
     const double v = V[idx] - mean[idx % S_BLK];
@@ -728,8 +740,9 @@ __global__ void center_kernel(const double* __restrict__ V, const double* __rest
 
 // AtU[a][j] = sum_i A[i][a] u[i][j] in FP64: per-CTA partials (64 columns x
 // 4 row groups per CTA, all 16 j per thread), then a fixed-order sum over CTAs.
-__global__ void __launch_bounds__(256) atu_part_kernel(const float* __restrict__ A, const double* __restrict__ u, int n,
-                                                       int k, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) atu_part_kernel(const float* A, const double* u, int n,
+                                                       int k, double* part) {
+    pdl_begin();
     const int a = threadIdx.x % 64, rg = threadIdx.x / 64;
     double acc[S_BLK];
 #pragma unroll
@@ -737,12 +750,12 @@ __global__ void __launch_bounds__(256) atu_part_kernel(const float* __restrict__
     if (a < k) {
 #pragma unroll 4
         for (int i = blockIdx.x * 4 + rg; i < n; i += gridDim.x * 4) {
-            const double x = (double)__ldg(A + (size_t)i * k + a);
+            const double x = (double)*(A + (size_t)i * k + a);
             // the FP64 row of u (shared by the CTA's 64 columns): no conversions per product
             const double2* ur = reinterpret_cast<const double2*>(u + (size_t)i * S_BLK);
 #pragma unroll
             for (int q = 0; q < S_BLK / 2; ++q) {
-                const double2 v = __ldg(ur + q);
+                const double2 v = *(ur + q);
                 acc[2 * q] = fma(x, v.x, acc[2 * q]);
                 acc[2 * q + 1] = fma(x, v.y, acc[2 * q + 1]);
             }
@@ -808,7 +821,7 @@ void mstack_f32(const float* dA, const float* u32, int n, int k, float* Mpart, f
     const int gx = std::min(MSF_CTAS, (n + MS_ROWS - 1) / MS_ROWS);
     mstack_f32_kernel<<<dim3(gx, S_BLK), 256, 0, s>>>(dA, u32, n, k, Mpart);
     const int cnt = S_BLK * k * k;
-    part_sum_kernel<float><<<(unsigned)(((size_t)cnt * 32 + 255) / 256), 256, 0, s>>>(Mpart, gx, cnt, 1.0f, M);
+    launch_next(part_sum_kernel<float>, (unsigned)(((size_t)cnt * 32 + 255) / 256), 256, 0, s, Mpart, gx, cnt, 1.0f, M);
 }
 
 // T2[i][j] = a_i^T M_j a_i for 4 consecutive j per CTA (M slices in shared memory)
@@ -897,11 +910,12 @@ void quadform_f32(const float* dA, const float* M, int n, int k, float* T2, cuda
 }
 
 // W = T1 - T2/2 + c.u/2 with T1 = A (A^T u) (FP64 accumulation), before centring
-__global__ void __launch_bounds__(256) factor_combine_kernel(const float* __restrict__ A,
-                                                             const double* __restrict__ AtU,
-                                                             const float* __restrict__ T2,
-                                                             const double* __restrict__ u, int n, int k,
-                                                             double* __restrict__ W) {
+__global__ void __launch_bounds__(256) factor_combine_kernel(const float* A,
+                                                             const double* AtU,
+                                                             const float* T2,
+                                                             const double* u, int n, int k,
+                                                             double* W) {
+    pdl_begin();
     // one thread per row: the row of A is read once for all 16 columns and
     // for |a_i|^2; A^T u sits in shared memory
     __shared__ __align__(16) double s_atu[64 * S_BLK];
@@ -930,7 +944,7 @@ __global__ void __launch_bounds__(256) factor_combine_kernel(const float* __rest
             float4 q[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h)
-                q[h] = a + 4 * h < k ? __ldg(reinterpret_cast<const float4*>(arow + a) + h) : make_float4(0, 0, 0, 0);
+                q[h] = a + 4 * h < k ? *(reinterpret_cast<const float4*>(arow + a) + h) : make_float4(0, 0, 0, 0);
 #pragma unroll
             for (int h = 0; h < 4; ++h)
                 if (a + 4 * h < k) {
@@ -949,7 +963,8 @@ __global__ void __launch_bounds__(256) factor_combine_kernel(const float* __rest
     for (int j = 0; j < S_BLK; ++j) W[o + j] = t1[j] - 0.5 * (double)T2[o + j] + 0.5 * cc * u[o + j];
 }
 
-__global__ void subtract_mean_kernel(double* __restrict__ W, const double* __restrict__ mean, int n) {
+__global__ void subtract_mean_kernel(double* W, const double* mean, int n) {
+    pdl_begin();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)n * S_BLK) return;
     W[idx] -= mean[idx % S_BLK];
@@ -1039,12 +1054,12 @@ size_t factor_tc_at_bytes(int n, int k);
 
 namespace {
 void col_mean(const double* V, int n, double* part, double* mean, cudaStream_t s) {
-    colsum_part_kernel<<<RED_CTAS, 256, 0, s>>>(V, n, part);
-    part_sum_kernel<double><<<(S_BLK * 32 + 255) / 256, 256, 0, s>>>(part, RED_CTAS, S_BLK, 1.0 / (double)n, mean);
+    launch_next(colsum_part_kernel, RED_CTAS, 256, 0, s, V, n, part);
+    launch_next(part_sum_kernel<double>, (S_BLK * 32 + 255) / 256, 256, 0, s, part, RED_CTAS, S_BLK, 1.0 / (double)n, mean);
 }
 void at_u(const float* A, const double* u, int n, int k, double* part, double* AtU, cudaStream_t s) {
-    atu_part_kernel<<<RED_CTAS, 256, 0, s>>>(A, u, n, k, part);
-    part_sum_kernel<double><<<(k * S_BLK * 32 + 255) / 256, 256, 0, s>>>(part, RED_CTAS, k * S_BLK, 1.0, AtU);
+    launch_next(atu_part_kernel, RED_CTAS, 256, 0, s, A, u, n, k, part);
+    launch_next(part_sum_kernel<double>, (k * S_BLK * 32 + 255) / 256, 256, 0, s, part, RED_CTAS, k * S_BLK, 1.0, AtU);
 }
 }  // namespace
 
@@ -1079,7 +1094,7 @@ rfx_status launch_mds_factors(Ctx* c, const float* dA, int k, int ndim, int max_
     auto apply = [&](const double* V, double* W) -> rfx_status {
         const unsigned gr = (unsigned)(((size_t)n * S_BLK + 255) / 256);
         col_mean(V, n, part, mean, s);
-        center_kernel<<<gr, 256, 0, s>>>(V, mean, n, u, u32);
+        launch_next(center_kernel, gr, 256, 0, s, V, mean, n, u, u32);
         at_u(dA, u, n, k, part, AtU, s);
         if (tensor) {
             rfx_status st = launch_factor_ops_tc(c, dA, k, Aq, At, sA, u32, M, T2);
@@ -1089,9 +1104,9 @@ rfx_status launch_mds_factors(Ctx* c, const float* dA, int k, int ndim, int max_
             quadform_f32(dA, M, n, k, T2, s);
             c->launches += 2;
         }
-        factor_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(dA, AtU, T2, u, n, k, W);
+        launch_next(factor_combine_kernel, (n + 255) / 256, 256, 0, s, dA, AtU, T2, u, n, k, W);
         col_mean(W, n, part, mean, s);
-        subtract_mean_kernel<<<gr, 256, 0, s>>>(W, mean, n);
+        launch_next(subtract_mean_kernel, gr, 256, 0, s, W, mean, n);
         c->launches += 9;
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
@@ -1148,7 +1163,7 @@ rfx_status launch_factor_operator(Ctx* c, const float* dA, int k, const double* 
     if (!mean || !u || !u32 || !AtU || !M || !Mpart || !T2 || !part) return RFX_ERR_OOM;
     const unsigned gr = (unsigned)(((size_t)n * S_BLK + 255) / 256);
     col_mean(V, n, part, mean, s);
-    center_kernel<<<gr, 256, 0, s>>>(V, mean, n, u, u32);
+    launch_next(center_kernel, gr, 256, 0, s, V, mean, n, u, u32);
     at_u(dA, u, n, k, part, AtU, s);
     rfx_status st = RFX_OK;
     if (precision) {
@@ -1165,9 +1180,9 @@ rfx_status launch_factor_operator(Ctx* c, const float* dA, int k, const double* 
         quadform_f32(dA, M, n, k, T2, s);
     }
     if (st != RFX_OK) return st;
-    factor_combine_kernel<<<(n + 255) / 256, 256, 0, s>>>(dA, AtU, T2, u, n, k, W);
+    launch_next(factor_combine_kernel, (n + 255) / 256, 256, 0, s, dA, AtU, T2, u, n, k, W);
     col_mean(W, n, part, mean, s);
-    subtract_mean_kernel<<<gr, 256, 0, s>>>(W, mean, n);
+    launch_next(subtract_mean_kernel, gr, 256, 0, s, W, mean, n);
     RFX_CUDA(cudaGetLastError());
     RFX_CUDA(cudaStreamSynchronize(s));
     return RFX_OK;
@@ -1181,7 +1196,7 @@ rfx_status launch_outlier_scores(Ctx* c, const float* dA, int k, float* d_out) {
     double* apart = d.get<double>((size_t)256 * k * k);
     if (!AtA || !apart) return RFX_ERR_OOM;
     ata_kernel<<<dim3(256, (k * k + 255) / 256), 256, 0, s>>>(dA, n, k, apart);
-    part_sum_kernel<double><<<(k * k * 32 + 255) / 256, 256, 0, s>>>(apart, 256, k * k, 1.0, AtA);
+    launch_next(part_sum_kernel<double>, (k * k * 32 + 255) / 256, 256, 0, s, apart, 256, k * k, 1.0, AtA);
     RFX_CUDA(cudaFuncSetAttribute(outlier_raw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)outlier_smem(k)));
     outlier_raw_kernel<<<(n + OR_ROWS - 1) / OR_ROWS, 256, outlier_smem(k), s>>>(dA, AtA, n, k, d_out);
@@ -1233,8 +1248,8 @@ rfx_status launch_mds3d_full(Ctx* c, const float* dP, double* d_coords, double* 
     // rows past n of the block in fragment order stay zero
     RFX_CUDA(cudaMemsetAsync(Vf, 0, sizeof(double) * (size_t)npad * S_BLK, s));
     auto apply = [&](const double*, double* W) -> rfx_status {
-        dgemm_bv_kernel<<<dim3(nt, ksn), 128, DB_SMEM, s>>>(B, nt, Vf, n, kchunk, Wpart, c->d_err);
-        if (W) bv_reduce_kernel<<<(unsigned)(((size_t)n * S_BLK + 255) / 256), 256, 0, s>>>(Wpart, n, ksn, W);
+        launch_next(dgemm_bv_kernel, dim3(nt, ksn), 128, DB_SMEM, s, B, nt, Vf, n, kchunk, Wpart, c->d_err);
+        if (W) launch_next(bv_reduce_kernel, (unsigned)(((size_t)n * S_BLK + 255) / 256), 256, 0, s, Wpart, n, ksn, W);
         c->launches += W ? 2 : 1;
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
