@@ -496,8 +496,8 @@ predict_kernel(const float* __restrict__ X, int m, int ms, int p, int nclass, in
         for (int t = blockIdx.y * run + w / SW; t < t1; t += TW) {
             const int64_t o = offs[t];
             const int32_t* cgl = catgoleft ? catgoleft + o * maxcat : nullptr;
-            const int c = PLAIN ? (XT ? walk_predict_plain(xc, nclass, nodes + o, nodeclass + o, maxnode)
-                                      : walk_predict_plain(xg, nclass, nodes + o, nodeclass + o, maxnode))
+            const int c = PLAIN ? (XT ? walk_predict_plain<false>(xc, nclass, nodes + o, nodeclass + o, maxnode)
+                                      : walk_predict_plain<SW == 1>(xg, nclass, nodes + o, nodeclass + o, maxnode))
                           : XT ? walk_predict(xc, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode)
                              : walk_predict(xg, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode);
             if (c < 0) continue;
@@ -513,8 +513,11 @@ predict_kernel(const float* __restrict__ X, int m, int ms, int p, int nclass, in
     }
 }
 
-// The same with an atomic per walk, for more classes than shared memory holds.
+// The same with an atomic per walk: one tree and 256 samples per CTA (the tree's
+// top levels in L1 for all of them), for a few hundred samples, where the walks'
+// latency counts, and for more classes than shared memory holds.
 constexpr int PRED_THREADS = 256;
+template <bool PLAIN>
 __global__ void __launch_bounds__(PRED_THREADS)
 predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode,
                       const DNode* __restrict__ nodes, const int32_t* __restrict__ nodeclass,
@@ -524,8 +527,10 @@ predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int
     const int s = blockIdx.x * PRED_THREADS + threadIdx.x;
     if (s >= m) return;
     const int64_t o = offs[t];
-    const int c = walk_predict(GlobalRow{X + (size_t)s * p}, p, nclass, nodes + o, nodeclass + o, cat,
-                               catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
+    const GlobalRow xr{X + (size_t)s * p};
+    const int c = PLAIN ? walk_predict_plain<false>(xr, nclass, nodes + o, nodeclass + o, maxnode)
+                        : walk_predict(xr, p, nclass, nodes + o, nodeclass + o, cat,
+                                       catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
     if (c >= 0) atomicAdd(votes + (size_t)s * nclass + c, 1);
 }
 
@@ -685,13 +690,19 @@ rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
             return plain ? go(predict_kernel<16, 2, true, true>, 16, 2) : go(predict_kernel<16, 2, true, false>, 16, 2);
         return plain ? go(predict_kernel<16, 2, false, true>, 16, 2) : go(predict_kernel<16, 2, false, false>, 16, 2);
     }
-    if (row <= 96 * 1024)
+    // up to 256 rows a warp per tree and 32 rows; from 1,500 rows 128 rows and
+    // four trees at a time (2,500 rows / 1,000 trees 66 us, 74 with a warp per
+    // tree and 71 with a CTA per tree); between them a CTA per tree (600 rows:
+    // 35 us, 40 and 37)
+    if (m < 256 && row <= 96 * 1024)
         return plain ? go(predict_kernel<1, 8, false, true>, 1, 8) : go(predict_kernel<1, 8, false, false>, 1, 8);
+    if (m >= 1500 && 4 * row <= 96 * 1024)
+        return plain ? go(predict_kernel<4, 4, false, true>, 4, 4) : go(predict_kernel<4, 4, false, false>, 4, 4);
     RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
     dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, T);
-    predict_direct_kernel<<<grid, PRED_THREADS, 0, c->stream>>>(dX, m, c->p, nc, 2 * c->n + 1, c->d_nodes,
-                                                                c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft,
-                                                                c->maxcat, d_votes);
+    (plain ? predict_direct_kernel<true> : predict_direct_kernel<false>)<<<grid, PRED_THREADS, 0, c->stream>>>(
+        dX, m, c->p, nc, 2 * c->n + 1, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft, c->maxcat,
+        d_votes);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }

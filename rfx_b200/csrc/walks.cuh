@@ -307,18 +307,28 @@ __device__ __forceinline__ int walk_terminal_plain(const XR& xrow, const DNode* 
     return 0;
 }
 
-template <typename XR>
+// PF: both children are loaded with the feature value (in range: checked at
+// load), one round trip to memory per step instead of two, for calls too small
+// to hide them.
+template <bool PF, typename XR>
 __device__ __forceinline__ int walk_predict_plain(const XR& xrow, int nclass, const DNode* __restrict__ nodes,
                                                   const int32_t* __restrict__ nclass_of, int maxnode) {
     int cur = 0;
+    DNode nd = load_node_now(nodes, 0);
     for (int k = 0; k < maxnode; ++k) {
-        const DNode nd = load_node(nodes, cur);
         if (node_status(nd.meta) == -1) {
             const int c = __ldg(nclass_of + cur);
             return (c >= 0 && c < nclass) ? c : 0;
         }
+        DNode cl, cr;
+        if constexpr (PF) {
+            cl = load_node_now(nodes, nd.left);
+            cr = load_node_now(nodes, nd.right);
+        }
         cur = step_plain(nd, xrow(node_var(nd.meta)));
         if (cur < 0) return 0;
+        if constexpr (PF) nd = cur == nd.left ? cl : cr;
+        else nd = load_node_now(nodes, cur);
     }
     return -1;
 }

@@ -1,5 +1,6 @@
-"""Test-set votes at the edges of the prediction kernel's tiles (32 and 512
-samples, the transposed copy from 4,096 rows on) and its class limits (counts in
+"""Test-set votes at the edges of the prediction kernel's tiles (32 samples
+up to 256 rows, one tree per CTA up to 1,500, 128 and then 512 samples, the
+transposed copy from 4,096 rows on) and its class limits (counts in
 shared memory, an atomic per walk beyond), with and without a go-left table, on
 numeric and mixed-type tables with values outside the levels, against the oracle
 (exact votes)."""
@@ -28,7 +29,7 @@ def _check(X, y, Xt, T, c, cat=None, table=False):
     assert np.array_equal(got, orc.predict(Xt, f)[0])
 
 
-@pytest.mark.parametrize("m", [1, 31, 33, 511, 4095, 4096, 4609])
+@pytest.mark.parametrize("m", [1, 31, 33, 255, 256, 1499, 1500, 4095, 4096, 4609])
 @pytest.mark.parametrize("table", [False, True])
 def test_predict_rows(built, m, table):
     X, y = synth.mixed_cover(900 + m, seed=m)
