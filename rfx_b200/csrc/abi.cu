@@ -162,6 +162,18 @@ bool is_device_ptr(const void* p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Managed memory is written like device memory, but the host can read it
+// without a copy, so calls that return results there wait for them.
+bool is_managed_ptr(const void* p) {
+    cudaPointerAttributes a;
+    if (!p) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeManaged;
+}
+
 rfx_status check_device_errors(Ctx* c) {
     uint32_t bits = 0;
     RFX_CUDA(cudaMemcpy(&bits, c->d_err, sizeof(bits), cudaMemcpyDeviceToHost));
@@ -198,6 +210,7 @@ static rfx_status with_f64_out(Ctx* c, double* out, size_t len, const char* who,
         st = copy_out(c, out, d, sizeof(double) * len);
         if (st == RFX_OK) st = finish_host(c, true);
     }
+    if (is_managed_ptr(out)) cudaStreamSynchronize(c->stream);
     return st;
 }
 
@@ -732,7 +745,8 @@ rfx_status rfx_oob_summary(rfx_ctx* ctx, float* oob_error, int32_t* pred, float*
     if (st == RFX_OK && hp) st = copy_out(c, pred, d_p, sizeof(int32_t) * c->n);
     if (st == RFX_OK && hpr) st = copy_out(c, proba, d_pr, sizeof(float) * (size_t)c->n * c->nclass);
     if (st == RFX_OK) st = finish_host(c, he || hp || hpr);
-    if (!tmp.empty()) cudaStreamSynchronize(c->stream);
+    if (!tmp.empty() || is_managed_ptr(oob_error) || is_managed_ptr(pred) || is_managed_ptr(proba))
+        cudaStreamSynchronize(c->stream);
     for (void* d : tmp) cudaFree(d);
     return st;
 }
@@ -821,7 +835,9 @@ rfx_status rfx_casewise_votes(rfx_ctx* ctx, float* q, int32_t* nout) {
         any_host |= !is_device_ptr(nout);
         if ((st = copy_out(c, nout, c->d_nout, sizeof(int32_t) * (size_t)c->n))) return st;
     }
-    return finish_host(c, any_host);
+    st = finish_host(c, any_host);
+    if (is_managed_ptr(q) || is_managed_ptr(nout)) cudaStreamSynchronize(c->stream);
+    return st;
 }
 
 rfx_status rfx_proximity_upper_f64(rfx_ctx* ctx, double* S, size_t len) {

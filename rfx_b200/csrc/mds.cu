@@ -1197,8 +1197,9 @@ rfx_status launch_outlier_scores(Ctx* c, const float* dA, int k, float* d_out) {
     if (!AtA || !apart) return RFX_ERR_OOM;
     ata_kernel<<<dim3(256, (k * k + 255) / 256), 256, 0, s>>>(dA, n, k, apart);
     launch_next(part_sum_kernel<double>, (k * k * 32 + 255) / 256, 256, 0, s, apart, 256, k * k, 1.0, AtA);
-    RFX_CUDA(cudaFuncSetAttribute(outlier_raw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)outlier_smem(k)));
+    int dev_smem = 0;
+    RFX_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    if (rfx_status st = allow_dyn_smem(outlier_raw_kernel, dev_smem)) return st;
     outlier_raw_kernel<<<(n + OR_ROWS - 1) / OR_ROWS, 256, outlier_smem(k), s>>>(dA, AtA, n, k, d_out);
     c->launches += 3;
     RFX_CUDA(cudaGetLastError());

@@ -471,14 +471,13 @@ oob_summary_kernel(const TV* __restrict__ votes, const int32_t* __restrict__ nou
 // where one run holds all trees).  With one warp per tree and 32 samples the
 // smallest calls spread over the GPU; large ones take 512 samples, whose
 // features then stay in L1 over the run.  Walks are short here (a categorical
-// split ends most), so the bound was the L1 tag stage (one line per lane and
-// feature, 87 % busy): XT reads a transposed copy, one line for the lanes at a
-// node (a third of the accesses), PLAIN drops the tests the load has made.
-// m = 50,000 / 1,000 trees / p = 54: 0.98 -> 0.86 ms; now bound by divergence
-// (13 of 32 lanes active), not memory.
-template <int SW, int TW, bool XT, bool PLAIN>
+// split ends most); PLAIN drops the tests the load has made.  m = 50,000 /
+// 1,000 trees / p = 54: 1.02 ms with a CTA per tree and 256 samples, 0.92 so,
+// 0.85 with PLAIN (reading a transposed copy of the rows instead: 0.98 and
+// 0.86); bound by divergence (13 of 32 lanes active), not memory.
+template <int SW, int TW, bool PLAIN>
 __global__ void __launch_bounds__(SW * TW * 32)
-predict_kernel(const float* __restrict__ X, int m, int ms, int p, int nclass, int maxnode, int T, int run,
+predict_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode, int T, int run,
                const DNode* __restrict__ nodes, const int32_t* __restrict__ nodeclass,
                const int64_t* __restrict__ offs, const int32_t* __restrict__ cat,
                const int32_t* __restrict__ catgoleft, int maxcat, int32_t* __restrict__ votes) {
@@ -490,16 +489,13 @@ predict_kernel(const float* __restrict__ X, int m, int ms, int p, int nclass, in
     for (int e = threadIdx.x; e < cells; e += SW * TW * 32) s_votes[e] = 0;
     __syncthreads();
     if (s < m) {
-        const GlobalRow xg{X + (size_t)s * p};
-        const ColumnRow xc{X + s, (size_t)ms};
+        const GlobalRow xr{X + (size_t)s * p};
         const int t1 = min(T, (int)(blockIdx.y + 1) * run);
         for (int t = blockIdx.y * run + w / SW; t < t1; t += TW) {
             const int64_t o = offs[t];
             const int32_t* cgl = catgoleft ? catgoleft + o * maxcat : nullptr;
-            const int c = PLAIN ? (XT ? walk_predict_plain<false>(xc, nclass, nodes + o, nodeclass + o, maxnode)
-                                      : walk_predict_plain<SW == 1>(xg, nclass, nodes + o, nodeclass + o, maxnode))
-                          : XT ? walk_predict(xc, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode)
-                             : walk_predict(xg, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode);
+            const int c = PLAIN ? walk_predict_plain<SW == 1>(xr, nclass, nodes + o, nodeclass + o, maxnode)
+                                : walk_predict(xr, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode);
             if (c < 0) continue;
             if (TW == 1) s_votes[sl * nclass + c] += 1;
             else atomicAdd(s_votes + sl * nclass + c, 1);
@@ -532,19 +528,6 @@ predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int
                         : walk_predict(xr, p, nclass, nodes + o, nodeclass + o, cat,
                                        catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
     if (c >= 0) atomicAdd(votes + (size_t)s * nclass + c, 1);
-}
-
-// XT = X transposed (p x m, row stride ms).
-__global__ void __launch_bounds__(256)
-transpose_kernel(const float* __restrict__ X, int m, int p, int ms, float* __restrict__ XT) {
-    __shared__ float tile[32][33];
-    const int i0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8)
-        if (i0 + r < m && c0 + tx < p) tile[r][tx] = X[(size_t)(i0 + r) * p + c0 + tx];
-    __syncthreads();
-    for (int r = ty; r < 32; r += 8)
-        if (c0 + r < p && i0 + tx < m) XT[(size_t)(c0 + r) * ms + i0 + tx] = tile[tx][r];
 }
 
 }  // namespace
@@ -653,19 +636,6 @@ rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
     if (m == 0) return RFX_OK;
     const int T = c->T, nc = c->nclass;
     const size_t row = 32 * (size_t)nc * sizeof(int32_t);
-    const int ms = (m + 31) & ~31;
-    // from 4,096 rows on (and where 512 samples' counts fit) the features are
-    // read from a transposed copy (made here, 5 us at 50,000 x 54; without room
-    // for it from the rows): the lanes of a warp hold consecutive samples, so
-    // one line serves all lanes at a node
-    Scratch sc(c);
-    const bool large = m >= 4096 && 16 * row <= 96 * 1024;
-    float* XT = large ? sc.get<float>((size_t)ms * c->p) : nullptr;
-    if (XT) {
-        transpose_kernel<<<dim3((m + 31) / 32, (c->p + 31) / 32), 256, 0, c->stream>>>(dX, m, c->p, ms, XT);
-        RFX_CUDA(cudaGetLastError());
-        c->launches += 1;
-    }
     auto go = [&](auto kernel, int sw, int tw) -> rfx_status {
         // runs of trees: enough CTAs for about eight rounds over the SMs, each
         // warp at least one tree
@@ -676,28 +646,28 @@ rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
         const int runs = (T + run - 1) / run;
         if (runs > 1) RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
         const size_t smem = row * sw;
-        if (smem > 48 * 1024)
-            RFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024) {
+            int dev_smem = 0;
+            RFX_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+            if (rfx_status st = allow_dyn_smem(kernel, dev_smem)) return st;
+        }
         kernel<<<dim3(cols, runs), sw * tw * 32, smem, c->stream>>>(
-            XT ? XT : dX, m, ms, c->p, nc, 2 * c->n + 1, T, run, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat,
+            dX, m, c->p, nc, 2 * c->n + 1, T, run, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat,
             c->d_catgoleft, c->maxcat, d_votes);
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
     };
     const bool plain = c->plain_walks;
-    if (large) {
-        if (XT)
-            return plain ? go(predict_kernel<16, 2, true, true>, 16, 2) : go(predict_kernel<16, 2, true, false>, 16, 2);
-        return plain ? go(predict_kernel<16, 2, false, true>, 16, 2) : go(predict_kernel<16, 2, false, false>, 16, 2);
-    }
-    // up to 256 rows a warp per tree and 32 rows; from 1,500 rows 128 rows and
+    if (m >= 4096 && 16 * row <= 96 * 1024)
+        return plain ? go(predict_kernel<16, 2, true>, 16, 2) : go(predict_kernel<16, 2, false>, 16, 2);
+    // up to 255 rows a warp per tree and 32 rows; from 1,500 rows 128 rows and
     // four trees at a time (2,500 rows / 1,000 trees 66 us, 74 with a warp per
     // tree and 71 with a CTA per tree); between them a CTA per tree (600 rows:
     // 35 us, 40 and 37)
     if (m < 256 && row <= 96 * 1024)
-        return plain ? go(predict_kernel<1, 8, false, true>, 1, 8) : go(predict_kernel<1, 8, false, false>, 1, 8);
+        return plain ? go(predict_kernel<1, 8, true>, 1, 8) : go(predict_kernel<1, 8, false>, 1, 8);
     if (m >= 1500 && 4 * row <= 96 * 1024)
-        return plain ? go(predict_kernel<4, 4, false, true>, 4, 4) : go(predict_kernel<4, 4, false, false>, 4, 4);
+        return plain ? go(predict_kernel<4, 4, true>, 4, 4) : go(predict_kernel<4, 4, false>, 4, 4);
     RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
     dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, T);
     (plain ? predict_direct_kernel<true> : predict_direct_kernel<false>)<<<grid, PRED_THREADS, 0, c->stream>>>(

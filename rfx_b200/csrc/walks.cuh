@@ -52,12 +52,6 @@ struct GlobalRow {
     const float* r;
     __device__ __forceinline__ float operator()(int m) const { return __ldg(r + m); }
 };
-// One sample's column of a feature-major table (row stride ms).
-struct ColumnRow {
-    const float* c;
-    size_t ms;
-    __device__ __forceinline__ float operator()(int m) const { return __ldg(c + m * ms); }
-};
 struct SharedRow {
     const float* r;
     __device__ __forceinline__ float operator()(int m) const { return r[m]; }

@@ -21,10 +21,10 @@
 //   id matches, the root included.
 //
 // Every float and double sum runs in the reference's order, so the results
-// are bit-identical to it: the pair-sum rows add tree after tree (a CTA
-// barrier between trees orders the adds into a column slot; within one tree a
-// row meets each column at most once), votes and qimp/qimpm loop over trees
-// in order per sample, rightimp loops over a tree's OOB samples in order.
+// are bit-identical to it: one warp owns a row's window and adds tree after
+// tree (within one tree a row meets each column at most once, so its lanes
+// never share a slot), votes and qimp/qimpm loop over trees in order per
+// sample, rightimp loops over a tree's OOB samples in order.
 #include <cuda_runtime.h>
 
 #include <algorithm>

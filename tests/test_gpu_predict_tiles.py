@@ -1,6 +1,6 @@
 """Test-set votes at the edges of the prediction kernel's tiles (32 samples
-up to 256 rows, one tree per CTA up to 1,500, 128 and then 512 samples, the
-transposed copy from 4,096 rows on) and its class limits (counts in
+below 256 rows, one tree per CTA below 1,500, 128 and from 4,096 rows on 512
+samples) and its class limits (counts in
 shared memory, an atomic per walk beyond), with and without a go-left table, on
 numeric and mixed-type tables with values outside the levels, against the oracle
 (exact votes)."""
