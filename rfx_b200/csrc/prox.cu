@@ -1060,13 +1060,10 @@ __device__ __forceinline__ double fp_value(double s, double inv_i, double inv_j)
     return __dmul_rn(0.5, __dadd_rn(__dmul_rn(h, inv_i), __dmul_rn(h, inv_j)));
 }
 
-// 1/nout per sample, formed once per call (1.0 where nout == 0).
-__global__ void finish_inv_kernel(const int32_t* __restrict__ nout, int n, double* __restrict__ inv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const int ni = nout[i];
-        inv[i] = ni > 0 ? __ddiv_rn(1.0, (double)ni) : 1.0;
-    }
+// 1/nout of a sample (1.0 where nout == 0).
+__device__ __forceinline__ double finish_inv(const int32_t* __restrict__ nout, int i) {
+    const int ni = __ldg(nout + i);
+    return ni > 0 ? __ddiv_rn(1.0, (double)ni) : 1.0;
 }
 
 // One CTA per tile of TR rows x TC columns at or right of the diagonal: the S
@@ -1078,12 +1075,14 @@ __global__ void finish_inv_kernel(const int32_t* __restrict__ nout, int n, doubl
 // pair for the full matrix); rows of an odd n start anywhere, so a tile's rows
 // and its mirror's are pieces of 512 and 256 bytes.  Tiles right of the
 // diagonal and inside the matrix run without a test per entry (1.35 -> 1.21
-// ms).
+// ms).  The tile's 1/nout are formed under its copies, one thread each (a table
+// made by a kernel before: 1.22 ms, and n = 501 / 5,001 11 / 41 us against 6.4 /
+// 36; every thread its own columns' instead: 1.30 ms).
 // Grid: y = pair of tile rows (I, nI - 1 - I), whose tile counts add up to
 // about the same, x = tile within the pair; CTAs of neighbouring columns run
 // together.
-// n = 30,001, full: 1.21 ms, 4.45 TB/s, 69 % of the measured copy rate; packed
-// 0.62 ms, 5.76 TB/s (before, one 32 x 32 tile at a time, four loads in flight per
+// n = 30,001, full: 1.20 ms, 4.50 TB/s, 70 % of the measured copy rate; packed
+// 0.62 ms, 5.79 TB/s (before, one 32 x 32 tile at a time, four loads in flight per
 // thread and two barriers per tile: 1.77 and 0.76 ms; a warp alone on 32-row
 // tiles with sixteen loads in flight: 2.79 ms).
 __host__ __device__ __forceinline__ int fp_tiles(int n, int I, int TR, int TC) {
@@ -1098,7 +1097,7 @@ __device__ __forceinline__ void fp_copy(void* dst, const void* src, int bytes) {
 
 // One tile; INNER: TR x TC entries, all right of the diagonal.
 template <typename TS, bool FULL, int TR, int TC, int FP_WARPS, bool INNER>
-__device__ __forceinline__ void finishprox_tile(const TS* __restrict__ S, const double* __restrict__ inv, int n,
+__device__ __forceinline__ void finishprox_tile(const TS* __restrict__ S, const int32_t* __restrict__ nout, int n,
                                                 float* __restrict__ P, TS* tile, double* s_inv, int i0, int j0) {
     constexpr int LD = TC + 1;
     constexpr int CW = TC / 32;        // columns per lane
@@ -1123,12 +1122,16 @@ __device__ __forceinline__ void finishprox_tile(const TS* __restrict__ S, const 
             sp += step0 - FP_WARPS * (i0 + r);
         }
     }
-    if (threadIdx.x < TR) s_inv[threadIdx.x] = (int)threadIdx.x < rows ? __ldg(inv + i0 + threadIdx.x) : 1.0;
-    double inv_j[CW];
-#pragma unroll
-    for (int u = 0; u < CW; ++u) inv_j[u] = INNER || lane + 32 * u < cols ? __ldg(inv + j0 + lane + 32 * u) : 1.0;
+    static_assert(TR + TC <= FP_WARPS * 32);
+    if (threadIdx.x < TR + TC) {
+        const int e = threadIdx.x < TR ? i0 + threadIdx.x : j0 + (threadIdx.x - TR);
+        s_inv[threadIdx.x] = e < n ? finish_inv(nout, e) : 1.0;
+    }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+    double inv_j[CW];
+#pragma unroll
+    for (int u = 0; u < CW; ++u) inv_j[u] = s_inv[TR + lane + 32 * u];
     {
         float* pp = (FULL ? P + (size_t)(i0 + w) * n : P + b0) + j0 + lane;
 #pragma unroll
@@ -1170,10 +1173,10 @@ __device__ __forceinline__ void finishprox_tile(const TS* __restrict__ S, const 
 
 template <typename TS, bool FULL, int TR, int TC, int FP_WARPS>
 __global__ void __launch_bounds__(FP_WARPS * 32)
-finishprox_kernel(const TS* __restrict__ S, const double* __restrict__ inv, int n, float* __restrict__ P) {
+finishprox_kernel(const TS* __restrict__ S, const int32_t* __restrict__ nout, int n, float* __restrict__ P) {
     extern __shared__ __align__(16) unsigned char fp_smem[];
     TS* tile = reinterpret_cast<TS*>(fp_smem);
-    __shared__ double s_inv[TR];
+    __shared__ double s_inv[TR + TC];
     const int nI = (n + TR - 1) / TR;
     int I = blockIdx.y, q = blockIdx.x;
     const int ta = fp_tiles(n, I, TR, TC);
@@ -1184,9 +1187,9 @@ finishprox_kernel(const TS* __restrict__ S, const double* __restrict__ inv, int 
     }
     const int i0 = I * TR, j0 = (i0 / TC + q) * TC;
     if (j0 > i0 + TR - 1 && i0 + TR <= n && j0 + TC <= n)
-        finishprox_tile<TS, FULL, TR, TC, FP_WARPS, true>(S, inv, n, P, tile, s_inv, i0, j0);
+        finishprox_tile<TS, FULL, TR, TC, FP_WARPS, true>(S, nout, n, P, tile, s_inv, i0, j0);
     else
-        finishprox_tile<TS, FULL, TR, TC, FP_WARPS, false>(S, inv, n, P, tile, s_inv, i0, j0);
+        finishprox_tile<TS, FULL, TR, TC, FP_WARPS, false>(S, nout, n, P, tile, s_inv, i0, j0);
 }
 
 }  // namespace
@@ -1416,7 +1419,7 @@ rfx_status launch_pairs_pipeline_raw(const PairsRawArgs& a, cudaStream_t stream)
 
 namespace {
 template <typename TS, bool FULL, int TR, int TC, int FP_WARPS>
-rfx_status finishprox_launch(Ctx* c, const TS* dS, const double* inv, float* dP) {
+rfx_status finishprox_launch(Ctx* c, const TS* dS, float* dP) {
     const int n = c->n;
     const int nI = (n + TR - 1) / TR;
     int bx = 1;  // the most tiles of a pair of tile rows
@@ -1426,32 +1429,24 @@ rfx_status finishprox_launch(Ctx* c, const TS* dS, const double* inv, float* dP)
     }
     constexpr int smem = TR * (TC + 1) * (int)sizeof(TS);
     auto kernel = finishprox_kernel<TS, FULL, TR, TC, FP_WARPS>;
-    RFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kernel<<<dim3(bx, (nI + 1) / 2), FP_WARPS * 32, smem, c->stream>>>(dS, inv, n, dP);
+    if (smem > 48 * 1024) RFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<dim3(bx, (nI + 1) / 2), FP_WARPS * 32, smem, c->stream>>>(dS, c->d_nout, n, dP);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }
 
 template <typename TS>
 rfx_status finishprox_run(Ctx* c, const TS* dS, float* dP, int full) {
-    StageTimer st(c, ST_FINISHPROX, 2);
-    Scratch sc(c);
+    StageTimer st(c, ST_FINISHPROX, 1);
     const int n = c->n;
-    double* inv = sc.get<double>((size_t)n);
-    if (!inv) {
-        set_error("finishprox: scratch allocation failed");
-        return RFX_ERR_OOM;
-    }
-    finish_inv_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(c->d_nout, n, inv);
-    RFX_CUDA(cudaGetLastError());
     // 64 x 128 tiles (33 KB, six CTAs an SM) once they fill the GPU, 64 x 64
     // below that (n = 30,001 full: 1.21 ms, 64 x 64 1.28, 128 x 128 1.21 but
     // 0.72 against 0.62 ms for the packed form)
     if (n >= 4096)
-        return full ? finishprox_launch<TS, true, 64, 128, 8>(c, dS, inv, dP)
-                    : finishprox_launch<TS, false, 64, 128, 8>(c, dS, inv, dP);
-    return full ? finishprox_launch<TS, true, 64, 64, 8>(c, dS, inv, dP)
-                : finishprox_launch<TS, false, 64, 64, 8>(c, dS, inv, dP);
+        return full ? finishprox_launch<TS, true, 64, 128, 8>(c, dS, dP)
+                    : finishprox_launch<TS, false, 64, 128, 8>(c, dS, dP);
+    return full ? finishprox_launch<TS, true, 64, 64, 8>(c, dS, dP)
+                : finishprox_launch<TS, false, 64, 64, 8>(c, dS, dP);
 }
 }  // namespace
 
