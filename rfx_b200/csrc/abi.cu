@@ -10,6 +10,7 @@
 #include <thread>
 #include <vector>
 
+#include "pointers.h"
 #include "rfx_internal.cuh"
 
 namespace rfxhost {
@@ -160,6 +161,16 @@ bool is_device_ptr(const void* p) {
         return false;
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+bool kernel_may_store(const Ctx* c, const void* p) {
+    if (!p) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return kernel_may_store(a, c->device);
 }
 
 // Managed memory is written like device memory, but the host can read it
@@ -665,10 +676,10 @@ rfx_status rfx_route_oob(rfx_ctx* ctx, int32_t* q, int32_t* nout, int32_t* leaf)
         set_error("rfx_route_oob: a case-wise context weighs the votes (float): use rfx_casewise_votes");
         return RFX_ERR_STATE;
     }
-    // device outputs are written by the routing itself, host ones copied out
-    const bool qdev = is_device_ptr(q), ndev = is_device_ptr(nout);
-    int32_t* dq = qdev ? q : nullptr;
-    int32_t* dn = ndev ? nout : nullptr;
+    // outputs in this device's memory are written by the routing itself, all
+    // others (host memory, another GPU's) copied out
+    int32_t* dq = kernel_may_store(c, q) ? q : nullptr;
+    int32_t* dn = kernel_may_store(c, nout) ? nout : nullptr;
     bool any_host = false;
     if (leaf) {
         int32_t* dleaf = leaf;
@@ -688,12 +699,12 @@ rfx_status rfx_route_oob(rfx_ctx* ctx, int32_t* q, int32_t* nout, int32_t* leaf)
     }
     c->routed = true;
     c->csr_built = false;
-    if (q && !qdev) {
-        any_host = true;
+    if (q && !dq) {
+        any_host |= !is_device_ptr(q);
         if ((st = copy_out(c, q, c->d_votes, sizeof(int32_t) * (size_t)c->n * c->nclass))) return st;
     }
-    if (nout && !ndev) {
-        any_host = true;
+    if (nout && !dn) {
+        any_host |= !is_device_ptr(nout);
         if ((st = copy_out(c, nout, c->d_nout, sizeof(int32_t) * (size_t)c->n))) return st;
     }
     return finish_host(c, any_host);

@@ -20,10 +20,18 @@ bool dev_or_null(const void* p) { return !p || is_device_ptr(p); }
 
 // One forest's analysis, enqueued on its context's stream with device outputs.
 rfx_status enqueue_item(Ctx* c, const rfx_batch_item& it) {
-    rfx_status st = launch_route(c, it.votes, it.nout);
+    int32_t* votes = kernel_may_store(c, it.votes) ? it.votes : nullptr;
+    int32_t* nout = kernel_may_store(c, it.nout) ? it.nout : nullptr;
+    rfx_status st = launch_route(c, votes, nout);
     if (st != RFX_OK) return st;
     c->routed = true;
     cudaStream_t s = c->stream;
+    // (on another GPU: copied)
+    if (it.votes && !votes)
+        RFX_CUDA(cudaMemcpyAsync(it.votes, c->d_votes, sizeof(int32_t) * (size_t)c->n * c->nclass,
+                                 cudaMemcpyDeviceToDevice, s));
+    if (it.nout && !nout)
+        RFX_CUDA(cudaMemcpyAsync(it.nout, c->d_nout, sizeof(int32_t) * c->n, cudaMemcpyDeviceToDevice, s));
     if (it.oob_error || it.oob_pred) {
         if ((st = launch_oob_summary(c, it.oob_error, it.oob_pred, nullptr)) != RFX_OK) return st;
     }

@@ -261,6 +261,7 @@ rfx_status dalloc(Ctx* c, T** p, size_t count) {
 }
 
 bool is_device_ptr(const void* p);
+bool kernel_may_store(const Ctx* c, const void* p);  // see pointers.h
 
 // Raise a kernel's dynamic shared-memory limit to everything the device allows
 // beside its static shared memory.  Setting the limit (not the launch's own
