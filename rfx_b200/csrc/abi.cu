@@ -189,7 +189,8 @@ rfx_status check_device_errors(Ctx* c) {
     uint32_t bits = 0;
     RFX_CUDA(cudaMemcpy(&bits, c->d_err, sizeof(bits), cudaMemcpyDeviceToHost));
     if (!bits) return RFX_OK;
-    RFX_CUDA(cudaMemset(c->d_err, 0, sizeof(uint32_t)));
+    RFX_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream));
+    RFX_CUDA(cudaStreamSynchronize(c->stream));
     std::string m = "device checks raised:";
     if (bits & ERR_STALE_JVR)
         m += " a cpu_testreeimp walk ended without a terminal node (the reference would keep a stale vote);";
@@ -260,13 +261,20 @@ rfx_status rfx_ctx_create(const rfx_config* cfg, rfx_ctx** out) {
     }
     rfx_status st = dalloc(c, &c->d_err, 1);
     if (st == RFX_OK) st = dalloc(c, &c->d_pairs, 4);
+    // cleared on the context's own stream: nothing orders another stream's work
+    // (the default stream's included) before what this one does next
+    if (st == RFX_OK) {
+        e = cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->d_pairs, 0, 4 * sizeof(unsigned long long), c->stream);
+        if (e != cudaSuccess) st = cuda_fail(e, "rfx_ctx_create");
+    }
     if (st != RFX_OK) {
+        if (c->d_err) cudaFree(c->d_err);
+        if (c->d_pairs) cudaFree(c->d_pairs);
         cudaStreamDestroy(c->stream);
         delete c;
         return st;
     }
-    cudaMemset(c->d_err, 0, sizeof(uint32_t));
-    cudaMemset(c->d_pairs, 0, 4 * sizeof(unsigned long long));
     *out = reinterpret_cast<rfx_ctx*>(c);
     return RFX_OK;
 }

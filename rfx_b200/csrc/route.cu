@@ -386,12 +386,14 @@ void route_launch(Ctx* c, int shape, int32_t* d_leaf) {
 // trees dealt over its warps (one thread per sample waited for T loads in a
 // few long chains: 51 us at n = 50,000 / 1,000 trees, 30 us this way).  Runs
 // after the walks: it also copies the finished votes and its counts to the
-// caller's device buffers (either may be null).
+// caller's device buffers (either may be null), and clears the three words that
+// the summary of these votes counts in.
 constexpr int NOUT_WARPS = 16;
 __global__ void __launch_bounds__(NOUT_WARPS * 32)
 nout_kernel(const uint8_t* __restrict__ inbag, int n, int T, int32_t* __restrict__ nout,
             const int32_t* __restrict__ votes, int nclass, int32_t* __restrict__ votes_out,
-            int32_t* __restrict__ nout_out) {
+            int32_t* __restrict__ nout_out, unsigned int* __restrict__ summary) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) summary[threadIdx.x] = 0u;
     __shared__ int s_c[NOUT_WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
@@ -419,8 +421,9 @@ nout_kernel(const uint8_t* __restrict__ inbag, int n, int T, int32_t* __restrict
 // reference's float arithmetic: argmax with >= (ties to the higher class),
 // total votes summed in float, probability = q / total (or 1/nclass).
 // The CTAs add their counts to counts[0..1]; the last one to finish (ticket
-// counts[2]) forms the error and leaves the three words zero for the next call.
-// One launch instead of a clear and two kernels.
+// counts[2]) forms the error and leaves the three words zero for another summary
+// of the same votes (nout_kernel has cleared them before the first).  One launch
+// instead of a clear and two kernels.
 template <typename TV>
 __global__ void __launch_bounds__(256)
 oob_summary_kernel(const TV* __restrict__ votes, const int32_t* __restrict__ nout, const int32_t* __restrict__ y,
@@ -532,9 +535,12 @@ predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int
 
 }  // namespace
 
+// The summary's words: they follow the pair counter.
+static unsigned int* summary_counts(Ctx* c) { return reinterpret_cast<unsigned int*>(c->d_pairs) + 2; }
+
 static rfx_status launch_nout(Ctx* c, int32_t* votes_out, int32_t* nout_out) {
     nout_kernel<<<(c->n + 31) / 32, NOUT_WARPS * 32, 0, c->stream>>>(c->d_inbag, c->n, c->T, c->d_nout, c->d_votes,
-                                                                     c->nclass, votes_out, nout_out);
+                                                                     c->nclass, votes_out, nout_out, summary_counts(c));
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }
@@ -615,9 +621,9 @@ rfx_status launch_route_leaf(Ctx* c, int32_t* d_leaf, int32_t* votes_out, int32_
 template <typename TV>
 static rfx_status oob_summary(Ctx* c, const TV* votes, float* d_errout, int32_t* d_pred, float* d_proba) {
     StageTimer st(c, ST_OOB, 1);
-    unsigned int* counts = reinterpret_cast<unsigned int*>(c->d_pairs) + 2;  // scratch words after the pair counter
     oob_summary_kernel<TV><<<(c->n + 255) / 256, 256, 0, c->stream>>>(votes, c->d_nout, c->d_y, c->n, c->nclass,
-                                                                      d_pred, d_proba, counts, d_errout);
+                                                                      d_pred, d_proba, summary_counts(c),
+                                                                      d_errout);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }

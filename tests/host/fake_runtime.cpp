@@ -220,8 +220,21 @@ static int other_gpu() {
     return q[5] == 5 ? 0 : fail("managed votes did not arrive");
 }
 
+// The error word and the counters are cleared in the order of the context's
+// stream: nothing may be left to a stream that does not order it.
+static int clears() {
+    rfx::Ctx* c = context(false);
+    if (!g_queue[nullptr].empty()) return fail("a new context leaves work on the default stream");
+    flush(c->stream);
+    if (*c->d_err || c->d_pairs[0] || c->d_pairs[1] || c->d_pairs[2]) return fail("a new context's words are not zero");
+    *c->d_err = 1;
+    if (rfx_synchronize(handle(c)) == RFX_OK) return fail("the error word was not read");
+    if (!g_queue[nullptr].empty() || !g_queue[c->stream].empty()) return fail("the clear is still to come");
+    return *c->d_err ? fail("the error word was not cleared") : 0;
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}};
+    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}, {"clears", clears}};
     const int rc = all.at(argv[argc - 1])();
     for (auto& f : g_faults) std::printf("%s\n", f.c_str());
     return g_faults.empty() ? rc : 1;
