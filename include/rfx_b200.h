@@ -6,9 +6,14 @@
  *
  * Every entry point returns an rfx_status (0 = success) and never throws.
  * Pointers are plain host or device pointers (the library inspects each one
- * with cudaPointerGetAttributes): outputs written to DEVICE memory are
- * enqueued on the context's stream and the call returns without waiting;
- * outputs written to HOST memory are complete when the call returns.
+ * with cudaPointerGetAttributes).  Outputs written to HOST memory are complete
+ * when the call returns.  Outputs written to DEVICE memory are complete too,
+ * except those of rfx_route_oob, rfx_proximity_upper_i32, rfx_finishprox and
+ * rfx_varimp: these calls enqueue their work on the context's stream and return
+ * without waiting, so a caller that reads such an output from another stream
+ * orders that stream after the context's (rfx_ctx_stream) or calls
+ * rfx_synchronize first.  The context's stream is a non-blocking one: the
+ * default stream is not ordered with it.
  * All output buffers are caller-allocated.
  *
  * Reference interfaces replaced (chriskuchar/RFX):

@@ -3,7 +3,11 @@ tests and bench.py use.  It is the kind of ctypes stub a maintainer of the
 reference would add to call the library from Python.
 
 Device outputs may be given as torch CUDA tensors (or raw device addresses);
-host outputs as numpy arrays.  There is no CPU fallback: if the library or a
+host outputs as numpy arrays.  With device outputs, ``route_oob``,
+``proximity_upper``, ``finishprox`` and ``varimp`` return while their work is
+still queued on the context's stream, which torch's streams are not ordered
+with: call ``synchronize`` (or wait for ``stream``) before reading them.  All
+other calls are complete on return.  There is no CPU fallback: if the library or a
 CUDA device is missing, every call raises.
 """
 from __future__ import annotations

@@ -173,18 +173,6 @@ bool kernel_may_store(const Ctx* c, const void* p) {
     return kernel_may_store(a, c->device);
 }
 
-// Managed memory is written like device memory, but the host can read it
-// without a copy, so calls that return results there wait for them.
-bool is_managed_ptr(const void* p) {
-    cudaPointerAttributes a;
-    if (!p) return false;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return a.type == cudaMemoryTypeManaged;
-}
-
 rfx_status check_device_errors(Ctx* c) {
     uint32_t bits = 0;
     RFX_CUDA(cudaMemcpy(&bits, c->d_err, sizeof(bits), cudaMemcpyDeviceToHost));
@@ -204,7 +192,8 @@ rfx_status check_device_errors(Ctx* c) {
 
 using namespace rfx;
 
-// Device or host FP64 output of n(n+1)/2 entries through pooled staging.
+// Device or host FP64 output of n(n+1)/2 entries through pooled staging;
+// complete on return wherever it lies.
 template <typename F>
 static rfx_status with_f64_out(Ctx* c, double* out, size_t len, const char* who, F&& fill) {
     const bool dev = is_device_ptr(out);
@@ -222,7 +211,7 @@ static rfx_status with_f64_out(Ctx* c, double* out, size_t len, const char* who,
         st = copy_out(c, out, d, sizeof(double) * len);
         if (st == RFX_OK) st = finish_host(c, true);
     }
-    if (is_managed_ptr(out)) cudaStreamSynchronize(c->stream);
+    cudaStreamSynchronize(c->stream);
     return st;
 }
 
@@ -764,8 +753,7 @@ rfx_status rfx_oob_summary(rfx_ctx* ctx, float* oob_error, int32_t* pred, float*
     if (st == RFX_OK && hp) st = copy_out(c, pred, d_p, sizeof(int32_t) * c->n);
     if (st == RFX_OK && hpr) st = copy_out(c, proba, d_pr, sizeof(float) * (size_t)c->n * c->nclass);
     if (st == RFX_OK) st = finish_host(c, he || hp || hpr);
-    if (!tmp.empty() || is_managed_ptr(oob_error) || is_managed_ptr(pred) || is_managed_ptr(proba))
-        cudaStreamSynchronize(c->stream);
+    cudaStreamSynchronize(c->stream);
     for (void* d : tmp) cudaFree(d);
     return st;
 }
@@ -855,7 +843,7 @@ rfx_status rfx_casewise_votes(rfx_ctx* ctx, float* q, int32_t* nout) {
         if ((st = copy_out(c, nout, c->d_nout, sizeof(int32_t) * (size_t)c->n))) return st;
     }
     st = finish_host(c, any_host);
-    if (is_managed_ptr(q) || is_managed_ptr(nout)) cudaStreamSynchronize(c->stream);
+    cudaStreamSynchronize(c->stream);
     return st;
 }
 

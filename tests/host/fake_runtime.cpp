@@ -233,8 +233,28 @@ static int clears() {
     return *c->d_err ? fail("the error word was not cleared") : 0;
 }
 
+// Calls that return their results complete, also in device memory.
+static int complete() {
+    rfx::Ctx* c = context(false);
+    auto* err = (float*)dev_int(1, 0);
+    int32_t* pred = dev_int(3, 0);
+    auto* d = (double*)dev_int(12, 0);
+    if (rfx_oob_summary(handle(c), err, pred, nullptr) != RFX_OK || pred[2] != 3) return fail("rfx_oob_summary");
+    if (rfx_proximity_upper_f64(handle(c), d, 6) != RFX_OK || ((int32_t*)d)[11] != 9) return fail("rfx_proximity_upper_f64");
+    d = (double*)dev_int(12, 0);
+    if (rfx_proximity_rfgap(handle(c), d, 6) != RFX_OK || ((int32_t*)d)[11] != 9) return fail("rfx_proximity_rfgap");
+    if (!g_queue[c->stream].empty()) return fail("work is left on the stream");
+    rfx::Ctx* cw = context(true);
+    int32_t *q = dev_int(6, 0), *nout = dev_int(3, 0), *pred2 = dev_int(3, 0);
+    if (rfx_casewise_votes(handle(cw), (float*)q, nout) != RFX_OK || q[5] != 7 || nout[2] != 4)
+        return fail("rfx_casewise_votes");
+    if (rfx_oob_summary(handle(cw), nullptr, pred2, nullptr) != RFX_OK || pred2[2] != 3)
+        return fail("rfx_oob_summary (case-wise)");
+    return g_queue[cw->stream].empty() ? 0 : fail("work is left on the stream");
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}, {"clears", clears}};
+    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}, {"clears", clears}, {"complete", complete}};
     const int rc = all.at(argv[argc - 1])();
     for (auto& f : g_faults) std::printf("%s\n", f.c_str());
     return g_faults.empty() ? rc : 1;
