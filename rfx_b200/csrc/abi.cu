@@ -910,15 +910,16 @@ rfx_status rfx_proximity_rfgap(rfx_ctx* ctx, double* P, size_t len) {
         set_error("rfx_proximity_rfgap: P must hold n(n+1)/2 entries");
         return RFX_ERR_INVALID;
     }
+    // node-id keys: 2 * nnode + 1 slots per tree (held here: the copy below reads
+    // the table up to the wait in with_f64_out)
+    const int T = c->T, n = c->n;
+    std::vector<int64_t> sb(T + 1, 0);
+    for (int t = 0; t < T; ++t) sb[t + 1] = sb[t] + 2 * (int64_t)c->h_nnode[t] + 1;
     return with_f64_out(c, P, len, "rfx_proximity_rfgap", [&](double* dP) -> rfx_status {
-        const int T = c->T, n = c->n;
         Scratch sc(c);
         int32_t* leaf = sc.get<int32_t>((size_t)T * n);
         int32_t* key = sc.get<int32_t>((size_t)T * n);
         int32_t* memb = sc.get<int32_t>((size_t)T * n);
-        // node-id keys: 2 * nnode + 1 slots per tree
-        std::vector<int64_t> sb(T + 1, 0);
-        for (int t = 0; t < T; ++t) sb[t + 1] = sb[t] + 2 * (int64_t)c->h_nnode[t] + 1;
         int64_t* dsb = sc.get<int64_t>((size_t)T + 1);
         int32_t* segoff = sc.get<int32_t>((size_t)sb[T]);
         if (!leaf || !key || !memb || !dsb || !segoff) {

@@ -30,6 +30,7 @@ std::map<void*, std::deque<Op>> g_queue;  // per stream; key nullptr: the legacy
 std::map<const char*, Range> g_mem;
 std::vector<std::string> g_faults;
 int g_copies = 0;
+bool g_running = false;  // within main
 rfx_status g_route_status = RFX_OK;
 
 Range where(const void* p) {
@@ -70,10 +71,11 @@ void kernel_store(rfx::Ctx* c, void* dst, size_t words, int32_t v) {
                                   nullptr});
 }
 
-bool reads_dead_memory() {
+// whether a queued copy still has to read from p
+bool source_of_a_copy(const void* p) {
     for (auto& q : g_queue)
         for (auto& op : q.second)
-            if (op.reads_host) return true;
+            if (p && op.reads_host == p) return true;
     return false;
 }
 
@@ -83,6 +85,16 @@ int fail(const char* what) {
 }
 
 }  // namespace
+
+// Host memory given back while a queued copy still reads it.
+void operator delete(void* p) noexcept {
+    if (g_running && source_of_a_copy(p)) {
+        std::fprintf(stderr, "host memory freed under a copy\n");
+        std::_Exit(1);
+    }
+    std::free(p);
+}
+void operator delete(void* p, size_t) noexcept { operator delete(p); }
 
 extern "C" {
 void** __cudaRegisterFatBinary(void*) { static void* h = nullptr; return &h; }
@@ -253,9 +265,21 @@ static int complete() {
     return g_queue[cw->stream].empty() ? 0 : fail("work is left on the stream");
 }
 
+// The key table of RF-GAP outlives its copy, also where a launch fails.
+static int tables() {
+    rfx::Ctx* c = context(false);
+    auto* d = (double*)dev_int(12, 0);
+    if (rfx_proximity_rfgap(handle(c), d, 6) != RFX_OK) return fail("rfx_proximity_rfgap");
+    g_route_status = RFX_ERR_CUDA;
+    if (rfx_proximity_rfgap(handle(c), d, 6) != RFX_ERR_CUDA) return fail("rfx_proximity_rfgap hides an error");
+    return 0;
+}
+
 int main(int argc, char** argv) {
-    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}, {"clears", clears}, {"complete", complete}};
+    const std::map<std::string, int (*)()> all = {{"other_gpu", other_gpu}, {"clears", clears}, {"complete", complete}, {"tables", tables}};
+    g_running = true;
     const int rc = all.at(argv[argc - 1])();
+    g_running = false;
     for (auto& f : g_faults) std::printf("%s\n", f.c_str());
     return g_faults.empty() ? rc : 1;
 }
