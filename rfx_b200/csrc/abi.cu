@@ -1328,10 +1328,14 @@ rfx_status rfx_factor_mds_operator(rfx_ctx* ctx, int use_quantized, int precisio
         cudaFree(dV);
         return cuda_fail(e, "rfx_factor_mds_operator");
     }
+    // (copies between device buffers return early, and the context's stream does
+    // not wait for the default stream's)
     e = cudaMemcpy(dV, V, sizeof(double) * cnt, cudaMemcpyDefault);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     st = e == cudaSuccess ? launch_factor_operator(c, dA, c->lr_rank, dV, dW, precision) : cuda_fail(e, "copy");
     if (st == RFX_OK) {
         e = cudaMemcpy(W, dW, sizeof(double) * cnt, cudaMemcpyDefault);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) st = cuda_fail(e, "copy");
     }
     cudaFree(dV);

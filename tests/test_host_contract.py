@@ -21,7 +21,7 @@ def program(built, tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["other_gpu", "clears", "complete", "tables"])
+@pytest.mark.parametrize("scenario", ["other_gpu", "clears", "complete", "tables", "operator_block"])
 def test_scenario(program, scenario):
     r = subprocess.run([program, scenario], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
