@@ -312,9 +312,10 @@ rfx_status rfx_graph_destroy(rfx_graph* g);
 /* Launch-shape autotuner (no counterpart in the reference).  The routing,
  * pair-count, varimp-walk, per-sample importance and low-rank leaf-sum stages
  * each offer a few launch shapes with identical results; the first run for a
- * problem shape (device and power-of-two buckets of n, ntree, p) runs each
- * once untimed, then times each once on the context stream and keeps the
- * fastest for the process.  Setting RFX_AUTOTUNE=0 keeps the default shapes,
+ * problem shape (device, power-of-two buckets of n, ntree, p, and the form of
+ * the stage's kernels: forests with or without a go-left table, low-rank rows
+ * of up to or over 128 entries) runs each once untimed, then times each once on
+ * the context stream and keeps the fastest for the process.  Setting RFX_AUTOTUNE=0 keeps the default shapes,
  * and RFX_TUNE_ROUTE / RFX_TUNE_PAIRS / RFX_TUNE_VWALK / RFX_TUNE_ROUTE_LEAF /
  * RFX_TUNE_PAIRS_HUB / RFX_TUNE_SEGSUM / RFX_TUNE_VSAMPLE = <shape> force one
  * shape; nothing is tuned while a stream is being captured.
@@ -322,7 +323,8 @@ rfx_status rfx_graph_destroy(rfx_graph* g);
  * 1 pair counts, 2 varimp walk, 3 routing in leaf order, 4 pair counts with
  * hub tiles, 5-7 low-rank leaf sums in FP32 / BF16 / FP8, 8 per-sample
  * importance sums), device, log2 n, log2 ntree, log2 p, shape}
- * and sets *count to the number of records. */
+ * and sets *count to the number of records (two of the same sizes where two
+ * forms were tuned). */
 rfx_status rfx_tuned_shapes(int32_t* out, int32_t cap, int32_t* count);
 
 /* Allocation-free pair counts.  No counterpart in the reference.

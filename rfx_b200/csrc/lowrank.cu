@@ -896,7 +896,7 @@ rfx_status apply_m(Ctx* c, const float* V, int w, float* MV, const float* dinv, 
             // shape 0: the warp takes the chunk's keys in turn; 1: slots of
             // the warp take several keys at once
             const int tk = is_fp8<TX>() ? TK_SEGSUM_FP8 : std::is_same<TX, float>::value ? TK_SEGSUM_F32 : TK_SEGSUM_BF16;
-            rfx_status st0 = autotune(c, tk, 2, 0, [&](int shape) -> rfx_status {
+            rfx_status st0 = autotune(c, tk, W > 128, 2, 0, [&](int shape) -> rfx_status {
                 if (shape == 1)
                     segsum_slot_kernel<TX, E, 4><<<nblk(chunks * 32), 256, 0, s>>>(
                         X, n, W, c->d_memb, c->d_segoff, c->d_segbase, t0, t1, cpt, gofs, G, Pf, Pl, fk, xs, gs);

@@ -1317,7 +1317,7 @@ rfx_status launch_pairs_upper(Ctx* c, int32_t* dS) {
         const int tk = hubs ? TK_PAIRS_HUB : TK_PAIRS16;
         const int nshape = PAIRS_SHAPES;
         const int defshape = hubs ? 1 : PAIRS_DEFAULT_SHAPE;
-        return autotune(c, tk, nshape, defshape, [&](int shape) -> rfx_status {
+        return autotune(c, tk, 0, nshape, defshape, [&](int shape) -> rfx_status {
             // the pair counter restarts from the hub leaves' pair updates
             if (hubs)
                 RFX_CUDA(cudaMemcpyAsync(c->d_pairs, hub_pairs, sizeof(unsigned long long), cudaMemcpyDeviceToDevice,

@@ -562,7 +562,7 @@ rfx_status launch_route(Ctx* c, int32_t* votes_out, int32_t* nout_out) {
         if (rfx_status s0 = allow_dyn_smem(route_leaf_staged_kernel<64>, dev_smem)) return s0;
         if (rfx_status s0 = allow_dyn_smem(route_leaf_staged_kernel<128>, dev_smem)) return s0;
         if (rfx_status s0 = allow_dyn_smem(route_leaf_staged_kernel<256>, dev_smem)) return s0;
-        r = autotune(c, TK_ROUTE_LEAF, 9, 1, [&](int shape) -> rfx_status {
+        r = autotune(c, TK_ROUTE_LEAF, c->plain_walks, 9, 1, [&](int shape) -> rfx_status {
             RFX_CUDA(cudaMemsetAsync(c->d_votes, 0, sizeof(int32_t) * (size_t)c->n * c->nclass, c->stream));
             auto go = [&](auto kernel, int rt, size_t smem) {
                 dim3 grid((c->n + rt - 1) / rt, c->T);
@@ -598,7 +598,7 @@ rfx_status launch_route(Ctx* c, int32_t* votes_out, int32_t* nout_out) {
             return RFX_OK;
         });
     } else {
-        r = autotune(c, TK_ROUTE, ROUTE_SHAPES, 0, [&](int shape) -> rfx_status {
+        r = autotune(c, TK_ROUTE, c->plain_walks, ROUTE_SHAPES, 0, [&](int shape) -> rfx_status {
             RFX_CUDA(cudaMemsetAsync(c->d_votes, 0, sizeof(int32_t) * (size_t)c->n * c->nclass, c->stream));
             route_launch(c, shape, nullptr);
             RFX_CUDA(cudaGetLastError());

@@ -1,7 +1,7 @@
 // Launch-shape autotuner.  A tunable stage offers a few launch shapes that
 // all compute the same result; the first time a stage runs for a given
-// problem shape (device, kernel, and power-of-two buckets of n, ntree and p)
-// each shape is run once untimed and once timed with CUDA events on the
+// problem shape (device, kernel, power-of-two buckets of n, ntree and p, and the
+// form of the kernels that the forest or the row width selects) each shape is run once untimed and once timed with CUDA events on the
 // context stream, the fastest is remembered for the rest of the process, and the stage's
 // result is the one the last timed run left behind (every shape writes the
 // complete result).  Tuning is skipped, and the default shape used, while the
@@ -29,7 +29,7 @@ int ilog2(long long v) {
 }
 
 std::mutex g_mu;
-std::map<std::tuple<int, int, int, int, int>, int> g_choice;
+std::map<std::tuple<int, int, int, int, int, int>, int> g_choice;
 
 bool tuning_enabled() {
     const char* e = std::getenv("RFX_AUTOTUNE");
@@ -51,10 +51,10 @@ int forced_shape(int kernel, int nvar) {
     return (v >= 0 && v < nvar) ? v : -1;
 }
 
-rfx_status autotune(Ctx* c, int kernel, int nvar, int def, const std::function<rfx_status(int)>& run) {
+rfx_status autotune(Ctx* c, int kernel, int form, int nvar, int def, const std::function<rfx_status(int)>& run) {
     const int forced = forced_shape(kernel, nvar);
     if (forced >= 0) return run(forced);
-    const auto key = std::make_tuple(kernel, c->device, ilog2(c->n), ilog2(c->T), ilog2(c->p));
+    const auto key = std::make_tuple(kernel, c->device, ilog2(c->n), ilog2(c->T), ilog2(c->p), form);
     {
         std::lock_guard<std::mutex> lk(g_mu);
         auto it = g_choice.find(key);

@@ -796,7 +796,7 @@ rfx_status launch_varimp_w(Ctx* c, int impn) {
         // shapes 0-2: rows through the read-only cache at 64/128/256 threads;
         // 3-5: the same with staged rows, where they fit in 96 KB; 6-8: rows
         // through the read-only cache with child-prefetching walks
-        rfx_status r = autotune(c, TK_VWALK, 9, 1, [&](int shape) -> rfx_status {
+        rfx_status r = autotune(c, TK_VWALK, c->plain_imp, 9, 1, [&](int shape) -> rfx_status {
             // the walk adds to the per-tree counts: clear them for every run
             RFX_CUDA(cudaMemsetAsync(c->d_right, 0, sizeof(int32_t) * 2 * (size_t)c->T, c->stream));
             RFX_CUDA(cudaMemsetAsync(c->d_rightimp, 0, sizeof(int32_t) * (size_t)c->T * c->p, c->stream));
@@ -843,7 +843,7 @@ rfx_status launch_varimp_w(Ctx* c, int impn) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         RFX_CUDA(cudaStreamIsCapturing(c->stream, &cap));
         const bool capturing = cap != cudaStreamCaptureStatusNone;
-        rfx_status r = autotune(c, TK_VSAMPLE, nshape, 0, [&](int shape) -> rfx_status {
+        rfx_status r = autotune(c, TK_VSAMPLE, 0, nshape, 0, [&](int shape) -> rfx_status {
             bool listed = false;
             if (shape == 1 && !capturing) {
                 // (where the lists do not fit in device memory the tree loop runs)
