@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <string>
 
 #include "walks.cuh"
@@ -737,16 +738,24 @@ rfx_status launch_casewise_votes(Ctx* c, const int32_t* d_leafnode, float* d_q) 
     return RFX_OK;
 }
 
+// Device bytes that a call's range table, and a chunk of trees' values in the
+// case-wise importance, may take; RFX_CW_MB (megabytes) overrides, e.g. to run
+// small forests in many pieces.
+static size_t piece_bytes() {
+    const char* e = std::getenv("RFX_CW_MB");
+    const long mb = e ? std::atol(e) : 0;
+    return (size_t)(mb > 0 ? mb : 256) << 20;
+}
+
 template <int MODE>
 static rfx_status weighted_rows(Ctx* c, const int32_t* key, const int64_t* segbase, const int32_t* segoff,
                                 const int32_t* memb, const long long* mass, double* out) {
     const int n = c->n, T = c->T;
-    // the range table holds as many rows as WR_TABLE bytes take (all rows of
+    // the range table holds as many rows as piece_bytes takes (all rows of
     // the sizes whose matrix fits easily), fewer where memory is short
-    constexpr size_t WR_TABLE = (size_t)256 << 20;
     Scratch sc(c);
     const size_t row_bytes = sizeof(WRange) * (size_t)T;
-    int rows = (int)std::min<size_t>((size_t)n, std::max<size_t>(32, WR_TABLE / row_bytes));
+    int rows = (int)std::min<size_t>((size_t)n, std::max<size_t>(32, piece_bytes() / row_bytes));
     WRange* tab = sc.get<WRange>((size_t)rows * T);
     while (!tab && rows > 1) {
         rows = (rows + 1) / 2;
@@ -756,7 +765,10 @@ static rfx_status weighted_rows(Ctx* c, const int32_t* key, const int64_t* segba
         set_error("weighted pair sums: scratch allocation failed");
         return RFX_ERR_OOM;
     }
-    double* wm = MODE == WR_PLAIN ? nullptr : sc.get<double>((size_t)n * T);
+    // member weights; RFX_CW_WEIGHTS=0 takes the form that runs without room for them
+    const char* pre = std::getenv("RFX_CW_WEIGHTS");
+    const bool per_pair = MODE == WR_PLAIN || (pre && std::string(pre) == "0");
+    double* wm = per_pair ? nullptr : sc.get<double>((size_t)n * T);
     if (wm) {
         member_weight_kernel<MODE><<<dim3((n + 255) / 256, T), 256, 0, c->stream>>>(key, segbase, segoff, memb, mass,
                                                                                     c->d_nin, n, wm);
@@ -815,12 +827,11 @@ rfx_status launch_gap_keys(Ctx* c, const int32_t* d_leafnode, int32_t* d_key) {
 rfx_status launch_casewise_varimp(Ctx* c, const int32_t* d_leafnode, int impn, float* d_avimp, float* d_sqsd,
                                   float* d_qimp, float* d_qimpm) {
     const int n = c->n, p = c->p, T = c->T;
-    // a chunk's values take at most CW_CHUNK bytes (one tree at least)
-    constexpr size_t CW_CHUNK = (size_t)256 << 20;
+    // a chunk's values take at most piece_bytes (one tree at least)
     Scratch sc(c);
     float* rr = sc.get<float>((size_t)T * p);
     const size_t per_tree = (size_t)n * (p + 1);
-    int chunk = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, CW_CHUNK / (per_tree * sizeof(float))));
+    int chunk = (int)std::min<size_t>((size_t)T, std::max<size_t>(1, piece_bytes() / (per_tree * sizeof(float))));
     chunk = std::min(chunk, 65535);  // grid y
     float* buf = rr ? sc.get<float>(per_tree * chunk) : nullptr;
     while (rr && !buf && chunk > 1) {
