@@ -281,7 +281,6 @@ __global__ void bv_reduce_kernel(const double* Wpart, int n, int ksn, double* W)
     W[idx] = a;
 }
 
-// G[S x S] += X^T Y over rows (atomics into a zeroed G).
 // Per-CTA partial Gram matrices X^T Y (16 x 16) into part[blockIdx.x], added
 // by gram_sum_kernel in a fixed order (reproducible run to run).
 __global__ void __launch_bounds__(256) dgram_kernel(const double* X, const double* Y, int n,
@@ -315,45 +314,18 @@ __global__ void gram_sum_kernel(const double* part, int nparts, double* G) {
     if (lane == 0) G[e] = v;
 }
 
-// Up to GRAM_FUSE partials (one load a lane) are added by the kernels below
-// themselves, in the same order, which saves the launch; more go through
-// gram_sum_kernel over the whole GPU first.
-constexpr int GRAM_FUSE = 32;
 constexpr int SMALL_THREADS = 512;
 
-// The 16 x 16 matrix into shared memory (leading dim ld): from G, or summed
-// from nparts <= GRAM_FUSE partials (a warp takes every 16th entry).
-__device__ __forceinline__ void load_gram(const double* G, const double* part, int nparts,
-                                          double* out, int ld) {
-    if (!part) {
-        for (int e = threadIdx.x; e < S_BLK * S_BLK; e += SMALL_THREADS) out[(e / S_BLK) * ld + e % S_BLK] = G[e];
-        return;
-    }
-    constexpr int NW = SMALL_THREADS / 32, PER = S_BLK * S_BLK / NW;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double v[PER];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) v[u] = lane < nparts ? part[(size_t)lane * (S_BLK * S_BLK) + w + u * NW] : 0.0;
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v[u] += __shfl_xor_sync(0xffffffffu, v[u], d);
-        const int e = w + u * NW;
-        if (lane == 0) out[(e / S_BLK) * ld + e % S_BLK] = v[u];
-    }
-}
-
 // One CTA: Cholesky of G and the inverse of its factor, T = L^{-T} (S x S).
-// A serial chain (16 square roots and divisions): 9.5 us from G, 15 us with
-// the sum of 32 partials (18 us, and 2 for the sum's own launch, with a dot
-// product per entry in one thread's chain).
-__global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* G,
-                                                                 const double* part, int nparts,
-                                                                 double* Tm, int* bad) {
+// A serial chain of 16 square roots and divisions (9.5 us).  The sum of the
+// partial Gram matrices stays a kernel of its own, also where there are few:
+// adding them here took 5.5 us, its launch takes less since it overlaps (whole
+// MDS at n = 2,000: 3.01 ms, 3.18 with the sum in here).
+__global__ void __launch_bounds__(SMALL_THREADS) chol_inv_kernel(const double* G, double* Tm, int* bad) {
     pdl_begin();
     __shared__ double L[S_BLK * S_BLK], Li[S_BLK * S_BLK];
     __shared__ double flag;
-    load_gram(G, part, nparts, L, S_BLK);
+    for (int e = threadIdx.x; e < S_BLK * S_BLK; e += SMALL_THREADS) L[e] = G[e];
     __syncthreads();
     if (!cta_cholesky_inverse(L, Li, S_BLK, S_BLK, &flag) && threadIdx.x == 0) *bad = 1;
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) {
@@ -389,18 +361,14 @@ __global__ void dright_kernel(const double* W, const double* Tm, int n,
 }
 
 // One CTA: eigen-decomposition of the S x S projection H (symmetrised).
-__global__ void __launch_bounds__(SMALL_THREADS) rr_kernel(const double* H,
-                                                           const double* part, int nparts,
-                                                           double* evals, double* evecs) {
+__global__ void __launch_bounds__(SMALL_THREADS) rr_kernel(const double* H, double* evals, double* evecs) {
     pdl_begin();
     constexpr int LD = S_BLK + 1;
-    __shared__ double Hs[S_BLK * S_BLK], A[S_BLK * LD], U[S_BLK * LD];
+    __shared__ double A[S_BLK * LD], U[S_BLK * LD];
     __shared__ int pairs[2 * 64];
-    load_gram(H, part, nparts, Hs, S_BLK);
-    __syncthreads();
     for (int e = threadIdx.x; e < S_BLK * S_BLK; e += blockDim.x) {
         const int i = e / S_BLK, j = e % S_BLK;
-        A[i * LD + j] = 0.5 * (Hs[i * S_BLK + j] + Hs[j * S_BLK + i]);
+        A[i * LD + j] = 0.5 * (H[i * S_BLK + j] + H[j * S_BLK + i]);
     }
     __syncthreads();
     cta_jacobi(A, U, S_BLK, LD, 30, pairs);
@@ -508,22 +476,20 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
         set_error("MDS: device allocation failed");
         return RFX_ERR_OOM;
     }
-    // Gram matrix of X and Y: partials, and their sum in G unless the kernel
-    // that reads it adds the few there are
-    const double* fuse = gb <= GRAM_FUSE ? gpart : nullptr;
+    // Gram matrix of X and Y in G
     auto gram = [&](const double* X, const double* Y) {
         launch_next(dgram_kernel, gb, 256, 0, s, X, Y, n, gpart);
-        if (!fuse) launch_next(gram_sum_kernel, S_BLK * S_BLK * 32 / 256, 256, 0, s, gpart, gb, G);
-        c->launches += fuse ? 1 : 2;
+        launch_next(gram_sum_kernel, S_BLK * S_BLK * 32 / 256, 256, 0, s, gpart, gb, G);
+        c->launches += 2;
     };
     // CholeskyQR2: Out = (src L1^{-T}) L2^{-T}, through the temporary Xt
     auto orth = [&](const double* src, double* Out) -> rfx_status {
         const unsigned gr = (unsigned)(((size_t)n * S_BLK + 255) / 256);
         gram(src, src);
-        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, Tm, bad);
+        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, Tm, bad);
         launch_next(dright_kernel, gr, 256, 0, s, src, Tm, n, Xt, nullptr);
         gram(Xt, Xt);
-        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, Tm, bad);
+        launch_next(chol_inv_kernel, 1, SMALL_THREADS, 0, s, G, Tm, bad);
         launch_next(dright_kernel, gr, 256, 0, s, Xt, Tm, n, Out, Vf);
         c->launches += 4;
         RFX_CUDA(cudaGetLastError());
@@ -537,7 +503,7 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
     // the k largest against the previous check into *delta
     auto ritz = [&](double* delta) -> rfx_status {
         gram(V, W);
-        launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, ev, U);
+        launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, ev, U);
         c->launches += 1;
         RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
         RFX_CUDA(cudaStreamSynchronize(s));
@@ -621,7 +587,7 @@ rfx_status subspace_topk(Ctx* c, int n, int k, Apply apply, int max_iter, double
         if (check) {
             // Rayleigh-Ritz on span(V): H = V^T (B V)
             gram(V, W);
-            launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, fuse, gb, ev, U);
+            launch_next(rr_kernel, 1, SMALL_THREADS, 0, s, G, ev, U);
             c->launches += 1;
             RFX_CUDA(cudaMemcpyAsync(cur.data(), ev, sizeof(double) * S_BLK, cudaMemcpyDeviceToHost, s));
             RFX_CUDA(cudaStreamSynchronize(s));
