@@ -738,11 +738,15 @@ inline size_t right_mul_smem(int w, int m) {
 }
 inline int right_mul_threads(int m) { return std::max(32, (RM_ROWS / 4) * (((m + 3) & ~3) / 4)); }
 
+// Leading dimension of the two arrays below: odd against bank conflicts, but at
+// w = 120 only rows of w fit a CTA's shared memory (227 KB).
+__host__ __device__ inline int eig_w_ld(int w) { return w < 120 ? w + 1 : w; }
+
 // One CTA: eigen-decomposition of the symmetrised w x w H.
 __global__ void __launch_bounds__(1024, 1) eig_w_kernel(const double* __restrict__ H, int w, double* __restrict__ evals,
                              double* __restrict__ evecs) {
-    extern __shared__ double sm[];  // two w x (w + 1) arrays
-    const int ld = w + 1;
+    extern __shared__ double sm[];  // two w x ld arrays
+    const int ld = eig_w_ld(w);
     double* A = sm;
     double* U = sm + w * ld;
     __shared__ int pairs[2 * 64];
@@ -942,7 +946,7 @@ rfx_status lowrank_compute(Ctx* c, int k, int oversample, int power_iters, int p
     cudaStream_t s = c->stream;
     const int n = c->n, T = c->T;
     const int w = (k + oversample + 7) / 8 * 8;  // rows of whole 16-byte chunks
-    if (k < 1 || w > 120 || w > n) {  // 120: two w x (w + 1) FP64 arrays in one CTA's shared memory
+    if (k < 1 || w > 120 || w > n) {  // 120: two w x w FP64 arrays in one CTA's shared memory
         set_error("rfx_lowrank: need 1 <= rank and rank + oversample (rounded up to a multiple of 8) <= min(120, n)");
         return RFX_ERR_INVALID;
     }
@@ -1057,7 +1061,7 @@ rfx_status lowrank_compute(Ctx* c, int k, int oversample, int power_iters, int p
     }
     const size_t sm2 = 2 * (size_t)w * w * sizeof(double);
     RFX_CUDA(cudaFuncSetAttribute(chol_inv_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2));
-    const size_t sm_eig = 2 * (size_t)w * (w + 1) * sizeof(double);
+    const size_t sm_eig = 2 * (size_t)w * eig_w_ld(w) * sizeof(double);
     RFX_CUDA(cudaFuncSetAttribute(eig_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_eig));
     RFX_CUDA(cudaFuncSetAttribute(right_mul_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)right_mul_smem(GW, GW)));

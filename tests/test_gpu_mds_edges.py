@@ -46,7 +46,7 @@ def test_full_matrix_mds(built, n):
     assert np.linalg.norm(B @ V - V * ev, axis=0).max() <= 1e-6 * w[0]
 
 
-@pytest.mark.parametrize("k", [1, 7, 63, 64, 65, 95])
+@pytest.mark.parametrize("k", [1, 7, 63, 64, 65, 95, 97, 104])
 def test_outlier_scores(built, k):
     n = 701  # the last CTA takes 29 of its 32 rows
     ctx = _load(n, 40, nodesize=5)
