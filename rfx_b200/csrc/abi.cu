@@ -520,6 +520,7 @@ static rfx_status load_forest(Ctx* c, const LoadInput& in) {
         }
         int most_levels = 0;
         for (int m = 0; m < p; ++m) most_levels = std::max(most_levels, in.cat[m]);
+        c->has_levels = levels;
         c->plain_walks = !in.has_catgoleft && most_levels <= (1 << 20) && c->max_nnode <= 2 * n + 1;
         c->plain_imp = !in.has_catgoleft && !herr.off_level;
         ALLOC(d_segoff, segbase[T]);

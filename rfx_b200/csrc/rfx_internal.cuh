@@ -66,6 +66,7 @@ struct Ctx {
     int max_keys = 0;                   // max_t 2*nleaf_t
     int max_nnode = 0;
     int iv_words = 0;                   // ceil(p / 64)
+    bool has_levels = false;            // some feature is categorical
     bool plain_walks = false;           // see walk_terminal_plain (walks.cuh)
     bool plain_imp = false;             // and every categorical training value rounds to 0..maxcat-1
 

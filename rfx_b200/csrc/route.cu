@@ -471,13 +471,8 @@ oob_summary_kernel(const TV* __restrict__ votes, const int32_t* __restrict__ nou
 // Test-set votes.  A CTA takes 32 SW samples and a run of trees, TW of them at
 // a time (warp w: samples 32 (w % SW) + lane, trees w / SW, w / SW + TW, ...),
 // counts in shared memory and adds each count to the votes once (or stores it,
-// where one run holds all trees).  With one warp per tree and 32 samples the
-// smallest calls spread over the GPU; large ones take 512 samples, whose
-// features then stay in L1 over the run.  Walks are short here (a categorical
-// split ends most); PLAIN drops the tests the load has made.  m = 50,000 /
-// 1,000 trees / p = 54: 1.02 ms with a CTA per tree and 256 samples, 0.92 so,
-// 0.85 with PLAIN (reading a transposed copy of the rows instead: 0.98 and
-// 0.86); bound by divergence (13 of 32 lanes active), not memory.
+// where one run holds all trees).  Walks are bound by latency and divergence,
+// not memory; PLAIN drops the tests the load has made.
 template <int SW, int TW, bool PLAIN>
 __global__ void __launch_bounds__(SW * TW * 32)
 predict_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode, int T, int run,
@@ -500,8 +495,7 @@ predict_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnod
             const int c = PLAIN ? walk_predict_plain<SW == 1>(xr, nclass, nodes + o, nodeclass + o, maxnode)
                                 : walk_predict(xr, p, nclass, nodes + o, nodeclass + o, cat, cgl, maxcat, maxnode);
             if (c < 0) continue;
-            if (TW == 1) s_votes[sl * nclass + c] += 1;
-            else atomicAdd(s_votes + sl * nclass + c, 1);
+            atomicAdd(s_votes + sl * nclass + c, 1);
         }
     }
     __syncthreads();
@@ -513,10 +507,8 @@ predict_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnod
 }
 
 // The same with an atomic per walk: one tree and 256 samples per CTA (the tree's
-// top levels in L1 for all of them), for a few hundred samples, where the walks'
-// latency counts, and for more classes than shared memory holds.
+// top levels in L1 for all of them).
 constexpr int PRED_THREADS = 256;
-template <bool PLAIN>
 __global__ void __launch_bounds__(PRED_THREADS)
 predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int maxnode,
                       const DNode* __restrict__ nodes, const int32_t* __restrict__ nodeclass,
@@ -526,10 +518,8 @@ predict_direct_kernel(const float* __restrict__ X, int m, int p, int nclass, int
     const int s = blockIdx.x * PRED_THREADS + threadIdx.x;
     if (s >= m) return;
     const int64_t o = offs[t];
-    const GlobalRow xr{X + (size_t)s * p};
-    const int c = PLAIN ? walk_predict_plain<false>(xr, nclass, nodes + o, nodeclass + o, maxnode)
-                        : walk_predict(xr, p, nclass, nodes + o, nodeclass + o, cat,
-                                       catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
+    const int c = walk_predict(GlobalRow{X + (size_t)s * p}, p, nclass, nodes + o, nodeclass + o, cat,
+                               catgoleft ? catgoleft + o * maxcat : nullptr, maxcat, maxnode);
     if (c >= 0) atomicAdd(votes + (size_t)s * nclass + c, 1);
 }
 
@@ -641,7 +631,6 @@ rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
     StageTimer st(c, ST_PREDICT, m > 0 ? 1 : 0);
     if (m == 0) return RFX_OK;
     const int T = c->T, nc = c->nclass;
-    const size_t row = 32 * (size_t)nc * sizeof(int32_t);
     auto go = [&](auto kernel, int sw, int tw) -> rfx_status {
         // runs of trees: enough CTAs for about eight rounds over the SMs, each
         // warp at least one tree
@@ -651,34 +640,46 @@ rfx_status launch_predict(Ctx* c, const float* dX, int m, int32_t* d_votes) {
         const int run = tw * ((per + std::min(want, per) - 1) / std::min(want, per));
         const int runs = (T + run - 1) / run;
         if (runs > 1) RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
-        const size_t smem = row * sw;
-        if (smem > 48 * 1024) {
-            int dev_smem = 0;
-            RFX_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-            if (rfx_status st = allow_dyn_smem(kernel, dev_smem)) return st;
-        }
+        const size_t smem = 32 * (size_t)sw * nc * sizeof(int32_t);  // at most 32 KB (512 rows, 16 classes)
         kernel<<<dim3(cols, runs), sw * tw * 32, smem, c->stream>>>(
             dX, m, c->p, nc, 2 * c->n + 1, T, run, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat,
             c->d_catgoleft, c->maxcat, d_votes);
         RFX_CUDA(cudaGetLastError());
         return RFX_OK;
     };
-    const bool plain = c->plain_walks;
-    if (m >= 4096 && 16 * row <= 96 * 1024)
-        return plain ? go(predict_kernel<16, 2, true>, 16, 2) : go(predict_kernel<16, 2, false>, 16, 2);
-    // up to 255 rows a warp per tree and 32 rows; from 1,500 rows 128 rows and
-    // four trees at a time (2,500 rows / 1,000 trees 66 us, 74 with a warp per
-    // tree and 71 with a CTA per tree); between them a CTA per tree (600 rows:
-    // 35 us, 40 and 37)
-    if (m < 256 && row <= 96 * 1024)
-        return plain ? go(predict_kernel<1, 8, true>, 1, 8) : go(predict_kernel<1, 8, false>, 1, 8);
-    if (m >= 1500 && 4 * row <= 96 * 1024)
-        return plain ? go(predict_kernel<4, 4, true>, 4, 4) : go(predict_kernel<4, 4, false>, 4, 4);
+    // A CTA per tree and 256 rows (direct) is the general form; votes in shared
+    // memory pay where their clear and sum are small beside the walks (few
+    // classes; at 40 they cost up to 40 %) and the rows' features then stay in L1.
+    // Plain walks pay where categorical splits end most walks, and with their
+    // prefetch in small calls on wide rows.  Device time at 1,000 trees, direct
+    // against the form taken (all forms, ten tables, 10 to 1,000 trees and 1 to
+    // 50,000 rows were timed; below the lines they are even or lose):
+    //   a few rows: 61 rows 18.3 -> 14.5 us (54 mixed features), 20.8 -> 15.2 (20
+    //   numeric); even at 300 trees;
+    //   categorical features: 2,000 rows 49.7 -> 45.7, 50,000 rows 968 -> 783;
+    //   with a go-left table 50,000 rows 925 -> 800, 4,000 rows even;
+    //   numeric: 8,000 rows of 40 features 244 -> 187, of 20 features 153 against
+    //   156; 50,000 rows of 20 features 938 -> 845, on trees of about 100 nodes 568
+    //   against 600, with 12 features and 10 classes 1,285 against 1,335.
+    const bool plain = c->plain_walks, wide = c->p >= 40;
+    const int64_t walks = (int64_t)m * T;
+    if (m < 256) {
+        if (plain && wide && nc <= 10) return go(predict_kernel<1, 8, true>, 1, 8);
+        if (nc <= 10 && (c->has_levels ? T >= 640 && m > 32 : T >= 480)) return go(predict_kernel<1, 8, false>, 1, 8);
+    } else if (c->has_levels) {
+        if (nc <= 16 && m >= 4096 && walks >= (plain ? 2000000 : 6000000))
+            return plain ? go(predict_kernel<16, 2, true>, 16, 2) : go(predict_kernel<16, 2, false>, 16, 2);
+        if (nc <= 16 && plain && m >= 1500 && T >= 640) return go(predict_kernel<4, 4, true>, 4, 4);
+    } else {
+        if (nc <= 16 && wide && m >= 1500 && (m < 32768 || c->p >= 80)) return go(predict_kernel<1, 8, false>, 1, 8);
+        if (m >= 32768 && nc <= (wide ? 10 : 5) && c->N >= 256 * (int64_t)T)
+            return go(predict_kernel<16, 2, false>, 16, 2);
+    }
     RFX_CUDA(cudaMemsetAsync(d_votes, 0, sizeof(int32_t) * (size_t)m * nc, c->stream));
-    dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, T);
-    (plain ? predict_direct_kernel<true> : predict_direct_kernel<false>)<<<grid, PRED_THREADS, 0, c->stream>>>(
-        dX, m, c->p, nc, 2 * c->n + 1, c->d_nodes, c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft, c->maxcat,
-        d_votes);
+    const dim3 grid((m + PRED_THREADS - 1) / PRED_THREADS, T);
+    predict_direct_kernel<<<grid, PRED_THREADS, 0, c->stream>>>(dX, m, c->p, nc, 2 * c->n + 1, c->d_nodes,
+                                                                c->d_nodeclass, c->d_offs, c->d_cat, c->d_catgoleft,
+                                                                c->maxcat, d_votes);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
 }
