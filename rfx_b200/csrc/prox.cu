@@ -149,13 +149,11 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
     }
     __syncthreads();
     // stable scatter: batch r * CSR_WARPS + w of 32 * CSR_GROUPS samples is
-    // warp w's in round r
+    // warp w's in round r; a turn per batch that holds samples
     const unsigned below = (1u << lane) - 1u;
     volatile uint8_t* tag = s_tag[w];
     constexpr int BATCH = 32 * CSR_GROUPS;
-    const int rounds = (n + BATCH * CSR_WARPS - 1) / (BATCH * CSR_WARPS);
-    for (int rd = 0; rd < rounds; ++rd) {
-        const int base = (rd * CSR_WARPS + w) * BATCH;
+    for (int base = w * BATCH; base < n; base += CSR_WARPS * BATCH) {
         // slot per sample: its key, K for key -1, K + 1 past the end
         int kv[CSR_GROUPS];
 #pragma unroll
@@ -185,8 +183,8 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
             }
             __syncwarp();
         }
-        // turn: after the warp before (and, for warp 0, the last warp of the round before)
-        if (w > 0 || rd > 0) csr_turn_wait(1 + w);
+        // turn: after the batch before, which the warp before has (warp 0: the last one)
+        if (base > 0) csr_turn_wait(1 + w);
         int start[CSR_GROUPS];
 #pragma unroll
         for (int u = 0; u < CSR_GROUPS; ++u) {
@@ -195,7 +193,7 @@ build_csr_kernel(const int32_t* __restrict__ key, int n, const int64_t* __restri
             if (kv[u] <= K && (grp[u] >> lane) == 1u) ctr.set(kv[u], start[u] + __popc(grp[u]));  // the slot's last lane
             __syncwarp();
         }
-        if (w + 1 < CSR_WARPS || rd + 1 < rounds) csr_turn_pass(w + 1 < CSR_WARPS ? 2 + w : 1);
+        if (base + BATCH < n) csr_turn_pass(w + 1 < CSR_WARPS ? 2 + w : 1);
 #pragma unroll
         for (int u = 0; u < CSR_GROUPS; ++u)
             if (kv[u] <= K) mt[start[u] + __popc(grp[u] & below)] = base + u * 32 + lane;
