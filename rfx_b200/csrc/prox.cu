@@ -1069,20 +1069,17 @@ __device__ __forceinline__ double finish_inv(const int32_t* __restrict__ nout, i
 // copies, so a tile's loads are all in flight with no registers held and any
 // alignment; every thread forms the values of the entries it copied, writes
 // them to the upper part and back into the tile, and the mirror goes out from
-// there (odd row stride: no bank conflicts).  DRAM bound (12 bytes per entry
-// pair for the full matrix); rows of an odd n start anywhere, so a tile's rows
-// and its mirror's are pieces of 512 and 256 bytes.  Tiles right of the
-// diagonal and inside the matrix run without a test per entry (1.35 -> 1.21
-// ms).  The tile's 1/nout are formed under its copies, one thread each (a table
-// made by a kernel before: 1.22 ms, and n = 501 / 5,001 11 / 41 us against 6.4 /
-// 36; every thread its own columns' instead: 1.30 ms).
+// there (odd row stride: no bank conflicts for INT32 sums, two-way ones for
+// FP64).  DRAM bound (12 bytes per entry pair for the full matrix of INT32 sums,
+// 16 of FP64); rows of an odd n start anywhere, so a tile's rows and its mirror's
+// are short unaligned pieces.  Tiles right of the diagonal and inside the matrix
+// run without a test per entry.  The tile's 1/nout are formed under its copies,
+// one thread each.
 // Grid: y = pair of tile rows (I, nI - 1 - I), whose tile counts add up to
 // about the same, x = tile within the pair; CTAs of neighbouring columns run
 // together.
-// n = 30,001, full: 1.20 ms, 4.50 TB/s, 70 % of the measured copy rate; packed
-// 0.62 ms, 5.79 TB/s (before, one 32 x 32 tile at a time, four loads in flight per
-// thread and two barriers per tile: 1.77 and 0.76 ms; a warp alone on 32-row
-// tiles with sixteen loads in flight: 2.79 ms).
+// n = 30,001, INT32: full 1.21 ms, 4.5 TB/s, 69 % of the measured copy rate,
+// packed 0.63 ms, 5.7 TB/s; FP64: full 1.37 ms (5.3 TB/s), packed 0.79 (6.8 TB/s).
 __host__ __device__ __forceinline__ int fp_tiles(int n, int I, int TR, int TC) {
     return (n + TC - 1) / TC - I * TR / TC;  // tiles of tile row I from the diagonal on
 }
@@ -1427,7 +1424,7 @@ rfx_status finishprox_launch(Ctx* c, const TS* dS, float* dP) {
     }
     constexpr int smem = TR * (TC + 1) * (int)sizeof(TS);
     auto kernel = finishprox_kernel<TS, FULL, TR, TC, FP_WARPS>;
-    if (smem > 48 * 1024) RFX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static_assert(smem <= 48 * 1024);
     kernel<<<dim3(bx, (nI + 1) / 2), FP_WARPS * 32, smem, c->stream>>>(dS, c->d_nout, n, dP);
     RFX_CUDA(cudaGetLastError());
     return RFX_OK;
@@ -1437,12 +1434,15 @@ template <typename TS>
 rfx_status finishprox_run(Ctx* c, const TS* dS, float* dP, int full) {
     StageTimer st(c, ST_FINISHPROX, 1);
     const int n = c->n;
-    // 64 x 128 tiles (33 KB, six CTAs an SM) once they fill the GPU, 64 x 64
-    // below that (n = 30,001 full: 1.21 ms, 64 x 64 1.28, 128 x 128 1.21 but
-    // 0.72 against 0.62 ms for the packed form)
-    if (n >= 4096)
-        return full ? finishprox_launch<TS, true, 64, 128, 8>(c, dS, dP)
-                    : finishprox_launch<TS, false, 64, 128, 8>(c, dS, dP);
+    // Tiles of 33 KB, six CTAs an SM.  INT32: 64 x 128 once they fill the GPU, 64 x
+    // 64 below (n = 30,001: full 1.21 ms, 64 x 64 1.27, packed 0.63 and 0.67; n =
+    // 2,001: 11.0 and 10.6 us, packed 10.7 and 9.2; even at 4,500).  FP64: 64 x 64
+    // at every size (64 x 128 takes 66 KB: n = 30,001 full 1.37 ms against 1.57,
+    // packed 0.79 against 1.11, n = 2,001 packed 9.8 us against 11.6).
+    if constexpr (sizeof(TS) == 4)
+        if (n >= 4096)
+            return full ? finishprox_launch<TS, true, 64, 128, 8>(c, dS, dP)
+                        : finishprox_launch<TS, false, 64, 128, 8>(c, dS, dP);
     return full ? finishprox_launch<TS, true, 64, 64, 8>(c, dS, dP)
                 : finishprox_launch<TS, false, 64, 64, 8>(c, dS, dP);
 }
