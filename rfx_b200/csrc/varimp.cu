@@ -221,8 +221,9 @@ joob_kernel(const uint8_t* __restrict__ inbag, int n, int32_t* __restrict__ joob
 // categorical split sends every walk right, so it is passed without a feature
 // value and cannot part the permuted walk from the path, and cpu_testreebag's
 // walk ends where the path ends (walked on its own only past an unsplit node or
-// the step guard).  Issue (55 %) and the L1 tag stage (66 %) share the bound;
-// n = 50,000 / 1,000 trees / p = 54 (44 of them 0/1): 2.19 ms (2.74 ms before).
+// the step guard).  Bound by the latency of dependent loads and the L1 stage
+// (66 % busy at n = 25,000); n = 50,000 / 1,000 trees / p = 54 (44 of them 0/1):
+// 2.19 ms (2.74 ms with the general walk).
 template <int W, int VW, bool FB = false, bool SX = false, bool PF = false, bool PLAIN = false>
 __global__ void __launch_bounds__(VW, (PF ? 1024 : 1536) / VW)  // PF: room for the children's registers
 varimp_walk_kernel(const float* __restrict__ X, const int32_t* __restrict__ y, int n, int p,
